@@ -27,7 +27,8 @@ u8p = np.ctypeslib.ndpointer(dtype=np.uint8, flags="C_CONTIGUOUS")
 def build() -> str:
     path = os.path.join(_HERE, "liboracle.so")
     subprocess.run(["make", "-s", "-C", _HERE], check=True)
-    if os.path.isdir(REFERENCE_ROOT):  # the reference's own helpers, where its sources are present
+    # the reference's own helpers, where its sources are present
+    if os.path.isfile(os.path.join(REFERENCE_ROOT, "SIMD_UAAMG", "levelset_util.cpp")):
         subprocess.run(["make", "-s", "-C", _HERE, "ref", f"REF={REFERENCE_ROOT}"], check=True)
     return path
 
