@@ -711,7 +711,7 @@ int uaamg_batch_destroy(uaamg_batch* b) {
     for (cudaEvent_t e : b->ev)
         if (e) cudaEventDestroy(e);
     if (b->ctx) {
-        if (b->dmem) cudaFreeAsync(b->dmem, b->stream);
+        ctx_dev_free(b->ctx, b->dmem, b->stream);
         if (b->stream != b->own_stream) cudaStreamSynchronize(b->stream);
         ctx_pinned_release(b->ctx, b->pin, b->pin_cap);
         ctx_stream_release(b->ctx, b->body_stream);

@@ -137,10 +137,10 @@ static void extrapolate_enqueue(DeviceCtx* ctx, cudaStream_t s, const HostMap& m
         }
         if (m0 != dmask) CK(cudaMemcpyAsync(dmask, m0, mb, cudaMemcpyDeviceToDevice, s));
     } catch (...) {
-        cudaFreeAsync(mem, s);
+        ctx_dev_free(ctx, mem, s);
         throw;
     }
-    CK(cudaFreeAsync(mem, s));
+    CK(ctx_dev_free(ctx, mem, s));
 }
 
 }  // namespace uaamg
@@ -173,11 +173,11 @@ int uaamg_extrapolate_channel(int n_layer, int64_t n_out, const int32_t* out_ori
         extrapolate_enqueue(ctx, s, map, n_layer, n_out, out_origins, dval, dmask, n_fill, fill_leaf, fill_masks);
         CK(cudaMemcpyAsync(values, dval, vb, cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(masks, dmask, mb, cudaMemcpyDeviceToHost, s));
-        CK(cudaFreeAsync(mem, s));
+        CK(ctx_dev_free(ctx, mem, s));
         mem = nullptr;
         CK(cudaStreamSynchronize(s));
     } catch (...) {
-        if (mem) cudaFreeAsync(mem, s);
+        ctx_dev_free(ctx, mem, s);
         cudaStreamSynchronize(s);
         ctx_stream_release(ctx, s);
         throw;

@@ -253,10 +253,10 @@ int uaamg_poisson_solve_fp64_reference(uaamg_poisson* h, const float* d_rhs, dou
             if (it > max_iter) it = max_iter;
         }
     } catch (...) {
-        cudaFreeAsync(mem, s);
+        ctx_dev_free(h->ctx, mem, s);
         throw;
     }
-    CK(cudaFreeAsync(mem, s));
+    CK(ctx_dev_free(h->ctx, mem, s));
     CK(cudaStreamSynchronize(s));
     if (iterations) *iterations = it;
     if (rel_residual) *rel_residual = rel;

@@ -82,7 +82,7 @@ static void mixed_free(uaamg_poisson* h) {
     MixedData* M = h->mixed;
     if (!M) return;
     mixed_destroy_graph(M);
-    if (M->mem) cudaFreeAsync(M->mem, h->stream);
+    ctx_dev_free(h->ctx, M->mem, h->stream);
     delete M;
     h->mixed = nullptr;
 }
@@ -529,7 +529,7 @@ int uaamg_poisson_true_residual_fp64(uaamg_poisson* h, const float* d_x, const f
     unsigned long long hb[2];
     CK(cudaMemcpyAsync(hb, buf, 16, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    if (!h->mixed) CK(cudaFreeAsync(buf, h->stream));
+    if (!h->mixed) CK(ctx_dev_free(h->ctx, buf, h->stream));
     memcpy(&out[0], &hb[0], 8);
     memcpy(&out[1], &hb[1], 8);
     return UAAMG_SUCCESS;

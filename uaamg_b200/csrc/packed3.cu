@@ -172,7 +172,7 @@ struct Packed3Call {
         CK(ctx_stream_acquire(ctx, &s));
     }
     ~Packed3Call() {
-        for (void* p : tofree) cudaFreeAsync(p, s);
+        for (void* p : tofree) ctx_dev_free(ctx, p, s);
         cudaStreamSynchronize(s);
         ctx_stream_release(ctx, s);
     }
@@ -222,7 +222,7 @@ int uaamg_packed3_from_vec3_device(const uaamg_leaf_grid* vec3, float* d_c0, flo
     std::vector<void*> tofree;
     float* dout[3] = {d_c0, d_c1, d_c2};
     packed3_split_dev(vec3, vec3->values, dout, ctx, s, tofree);
-    for (void* p : tofree) CK(cudaFreeAsync(p, s));
+    for (void* p : tofree) CK(ctx_dev_free(ctx, p, s));
     return UAAMG_SUCCESS;
     ABI_END
 }
@@ -309,7 +309,7 @@ int uaamg_packed3_to_vec3_device(const uaamg_leaf_grid* c0, const uaamg_leaf_gri
     std::vector<void*> tofree;
     const float* dval[3] = {c0->values, c1->values, c2->values};
     packed3_merge_dev(ch, dval, U, d_out_values, ctx, s, tofree);
-    for (void* p : tofree) CK(cudaFreeAsync(p, s));
+    for (void* p : tofree) CK(ctx_dev_free(ctx, p, s));
     return UAAMG_SUCCESS;
     ABI_END
 }

@@ -956,7 +956,7 @@ static void build_hierarchy(uaamg_poisson* h, const uaamg_leaf_grid* phi, const 
         }
         // the rhs and the velocities' buffers: done before the inputs are freed and the handle is used
         if (ri) CK(cudaStreamWaitEvent(s, ev_vel.e, 0));
-        for (void* pmem : tofree) CK(cudaFreeAsync(pmem, s));
+        for (void* pmem : tofree) CK(ctx_dev_free(h->ctx, pmem, s));
         tofree.clear();
         TRACE("coefficient kernels enqueued");
         h->nlev = nlev;
@@ -2013,8 +2013,10 @@ int uaamg_poisson_destroy(uaamg_poisson* h) {
     destroy_graph(h);
     if (h->ctx) mixed_free(h);
     if (h->ctx) {
-        if (h->dmem) cudaFreeAsync(h->dmem, h->stream);
-        if (h->dmem2) cudaFreeAsync(h->dmem2, h->stream);
+        // the handle's stream has been waited for; idle when its other streams have nothing left either
+        const bool idle = h->stream && h->body_stream && ctx_stream_idle(h->body_stream) && ctx_stream_idle(h->own_stream);
+        ctx_dev_free(h->ctx, h->dmem, h->stream, idle);
+        ctx_dev_free(h->ctx, h->dmem2, h->stream, idle);
         if (h->stream != h->own_stream) cudaStreamSynchronize(h->stream);
         ctx_pinned_release(h->ctx, h->pin_state, h->pin_state_cap);
         ctx_pinned_release(h->ctx, h->pin_stage, h->pin_stage_cap);
@@ -2094,7 +2096,7 @@ static int build_rhs_impl(uaamg_poisson* h, const uaamg_leaf_grid* fw, const uaa
     k_build_rhs<<<(unsigned)D0.L.nl, 128, 0, h->stream>>>(D0.L.mask, D0.org, g0.g, g1.g, g2.g, g3.g, g4.g, invdx, d_out);
     CHECK_LAUNCH();
     h->launches++;
-    for (void* p : tofree) CK(cudaFreeAsync(p, h->stream));
+    for (void* p : tofree) CK(ctx_dev_free(h->ctx, p, h->stream));
     return UAAMG_SUCCESS;
 }
 
@@ -2247,15 +2249,16 @@ struct Scratch {
     float* b = nullptr;
     float* c = nullptr;
     cudaStream_t s;
+    DeviceCtx* dc = nullptr;
     Scratch(size_t bytes, cudaStream_t st) : s(st) {
         cudaError_t ce = cudaSuccess;
-        DeviceCtx* dc = device_ctx(&ce);
+        dc = device_ctx(&ce);
         CK(ce);
         CK(ctx_dev_alloc(dc, (void**)&a, std::max<size_t>(bytes, 16) * 3, s));
         b = a + std::max<size_t>(bytes, 16) / 4;
         c = b + std::max<size_t>(bytes, 16) / 4;
     }
-    ~Scratch() { cudaFreeAsync(a, s); }
+    ~Scratch() { ctx_dev_free(dc, a, s); }
 };
 
 static void check_level(const uaamg_poisson* h, int level) {

@@ -262,7 +262,7 @@ static void face_weights_impl(const uaamg_leaf_grid* solid, int64_t n, const int
     if (masks) CK(cudaMemcpyAsync(dmask, masks, (size_t)n * 64, cudaMemcpyHostToDevice, s));
     k_face_weights<<<(unsigned)n, 128, 0, s>>>(g.g, dorg, dmask, (int)n, d_out);
     CHECK_LAUNCH();
-    for (void* p : tofree) CK(cudaFreeAsync(p, s));
+    for (void* p : tofree) CK(ctx_dev_free(ctx, p, s));
 }
 
 static void pressure_gradient_impl(uaamg_poisson* h, const uaamg_leaf_grid* phi, const uaamg_leaf_grid* fw,
@@ -310,7 +310,7 @@ static void pressure_gradient_impl(uaamg_poisson* h, const uaamg_leaf_grid* phi,
                                                     d_upd, d_refl, dt, h->lv[0].dx, friction);
     CHECK_LAUNCH();
     h->launches++;
-    for (void* p : tofree) CK(cudaFreeAsync(p, s));
+    for (void* p : tofree) CK(ctx_dev_free(h->ctx, p, s));
 }
 
 // immerse_liquid_phi_in_solids (FLIP_vdb/FLIP_vdb.cpp:2856-2942), the value
@@ -442,10 +442,10 @@ static void immerse_impl(const uaamg_leaf_grid* solid, const uaamg_leaf_grid* li
         k_immerse_solid<<<(unsigned)n, 128, 0, s>>>(gs.g, refg, dorg, dmask, (int)n, dx * 3.0f, d_out);
         CHECK_LAUNCH();
     } catch (...) {
-        for (void* p : tofree) cudaFreeAsync(p, s);
+        for (void* p : tofree) ctx_dev_free(ctx, p, s);
         throw;
     }
-    for (void* p : tofree) CK(cudaFreeAsync(p, s));
+    for (void* p : tofree) CK(ctx_dev_free(ctx, p, s));
 }
 
 }  // namespace
@@ -468,7 +468,7 @@ int uaamg_face_weights(const uaamg_leaf_grid* solid_sdf, int64_t leaf_count, con
         CK(ctx_dev_alloc(ctx, (void**)&d, bytes, s));
         face_weights_impl(solid_sdf, leaf_count, origins, masks, d, s);
         CK(cudaMemcpyAsync(weights, d, bytes, cudaMemcpyDeviceToHost, s));
-        CK(cudaFreeAsync(d, s));
+        CK(ctx_dev_free(ctx, d, s));
         CK(cudaStreamSynchronize(s));
     } catch (...) {
         cudaStreamSynchronize(s);
@@ -517,10 +517,10 @@ int uaamg_poisson_apply_pressure_gradient(uaamg_poisson* h, const uaamg_leaf_gri
         CK(cudaMemcpyAsync(mask_out, dmask, (size_t)n * 64, cudaMemcpyDeviceToHost, s));
         if (update_out) CK(cudaMemcpyAsync(update_out, dupd, vb, cudaMemcpyDeviceToHost, s));
         if (reflected_out) CK(cudaMemcpyAsync(reflected_out, drefl, vb, cudaMemcpyDeviceToHost, s));
-        CK(cudaFreeAsync(d, s));
+        CK(ctx_dev_free(h->ctx, d, s));
         CK(cudaStreamSynchronize(s));
     } catch (...) {
-        cudaFreeAsync(d, s);
+        ctx_dev_free(h->ctx, d, s);
         cudaStreamSynchronize(s);
         throw;
     }
@@ -563,11 +563,11 @@ int uaamg_immerse_liquid_phi(const uaamg_leaf_grid* solid_sdf, const uaamg_leaf_
         CK(ctx_dev_alloc(ctx, (void**)&d, bytes, s));
         immerse_impl(solid_sdf, liquid_phi, dx, d, s);
         CK(cudaMemcpyAsync(values_out, d, bytes, cudaMemcpyDeviceToHost, s));
-        CK(cudaFreeAsync(d, s));
+        CK(ctx_dev_free(ctx, d, s));
         d = nullptr;
         CK(cudaStreamSynchronize(s));
     } catch (...) {
-        if (d) cudaFreeAsync(d, s);
+        ctx_dev_free(ctx, d, s);
         cudaStreamSynchronize(s);
         ctx_stream_release(ctx, s);
         throw;

@@ -58,6 +58,11 @@ static float* srv_alloc(size_t bytes, cudaStream_t s) {
     CK(ctx_dev_alloc(ctx, &p, bytes, s));
     return reinterpret_cast<float*>(p);
 }
+static void srv_free(void* p, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    DeviceCtx* ctx = device_ctx(&e);
+    if (ctx) ctx_dev_free(ctx, p, s);
+}
 
 // A server-owned copy of an input grid.  Host grids are copied into host
 // memory, device grids into device memory (synchronously), so the caller may
@@ -75,7 +80,7 @@ struct SrvGrid {
     SrvGrid(const SrvGrid&) = delete;
     SrvGrid& operator=(const SrvGrid&) = delete;
     ~SrvGrid() {
-        if (dval) cudaFreeAsync(dval, stream);
+        if (dval) srv_free(dval, stream);
     }
     // `s`: the server's copy stream (device grids are copied on it, and it is
     // synchronised before the call returns)
@@ -190,9 +195,9 @@ static void srv_release_device(SrvReq& r, cudaStream_t s) {
     if (r.hv) uaamg_viscosity_destroy(r.hv);
     r.hp = nullptr;
     r.hv = nullptr;
-    if (r.dx_) cudaFreeAsync(r.dx_, s);
-    if (r.drhs) cudaFreeAsync(r.drhs, s);
-    if (r.dfw) cudaFreeAsync(r.dfw, s);
+    if (r.dx_) srv_free(r.dx_, s);
+    if (r.drhs) srv_free(r.drhs, s);
+    if (r.dfw) srv_free(r.dfw, s);
     r.dx_ = r.drhs = r.dfw = nullptr;
     if (r.lane_stream) cudaStreamDestroy(r.lane_stream);
     r.lane_stream = nullptr;

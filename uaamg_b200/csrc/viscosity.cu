@@ -340,7 +340,7 @@ static T* vupload(uaamg_viscosity* h, const T* src, size_t count) {
 static void vfree_now(uaamg_viscosity* h, void* p) {
     auto it = std::find(h->allocs.begin(), h->allocs.end(), p);
     if (it != h->allocs.end()) h->allocs.erase(it);
-    CK(cudaFreeAsync(p, h->stream));
+    CK(ctx_dev_free(h->ctx, p, h->stream));
 }
 static DMap vupload_map(uaamg_viscosity* h, const HostMap& m) {
     DMap d{};
@@ -1021,7 +1021,7 @@ static void vbuild_rhs_dev(uaamg_viscosity* h, const uaamg_leaf_grid* u, const u
     }
     CK(cudaStreamSynchronize(h->stream));
     while (h->allocs.size() > mark) {
-        CK(cudaFreeAsync(h->allocs.back(), h->stream));
+        CK(ctx_dev_free(h->ctx, h->allocs.back(), h->stream));
         h->allocs.pop_back();
     }
 }
@@ -1037,7 +1037,7 @@ static void vgather_dev(uaamg_viscosity* h, const uaamg_leaf_grid* u, const uaam
     launch2(k_vgather, dim3((unsigned)D.L.nl, 3), 128, h->stream, D.L, (const int*)D.org, U, d_out);
     CK(cudaStreamSynchronize(h->stream));
     while (h->allocs.size() > mark) {
-        CK(cudaFreeAsync(h->allocs.back(), h->stream));
+        CK(ctx_dev_free(h->ctx, h->allocs.back(), h->stream));
         h->allocs.pop_back();
     }
 }
@@ -1052,7 +1052,7 @@ struct VScratch {  // temporary device buffers of one host-pointer call
         return (float*)p;
     }
     ~VScratch() {
-        for (void* p : bufs) cudaFreeAsync(p, h->stream);
+        for (void* p : bufs) ctx_dev_free(h->ctx, p, h->stream);
     }
 };
 
@@ -1122,7 +1122,9 @@ int uaamg_viscosity_destroy(uaamg_viscosity* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     vdestroy_graph(h);
     if (h->ctx) {
-        for (void* p : h->allocs) cudaFreeAsync(p, h->stream);
+        // the handle's stream has been waited for; idle when its other streams have nothing left either
+        const bool idle = h->stream && h->body_stream && ctx_stream_idle(h->body_stream) && ctx_stream_idle(h->own_stream);
+        for (void* p : h->allocs) ctx_dev_free(h->ctx, p, h->stream, idle);
         h->allocs.clear();
         if (h->stream) cudaStreamSynchronize(h->stream);
         ctx_pinned_release(h->ctx, h->pin_state, h->pin_state_cap);
@@ -1285,13 +1287,13 @@ int uaamg_viscosity_solve_velocity(uaamg_viscosity* h, const uaamg_leaf_grid* u,
     } catch (...) {
         cudaStreamSynchronize(h->stream);
         while (h->allocs.size() > mark) {
-            cudaFreeAsync(h->allocs.back(), h->stream);
+            ctx_dev_free(h->ctx, h->allocs.back(), h->stream);
             h->allocs.pop_back();
         }
         throw;
     }
     while (h->allocs.size() > mark) {
-        CK(cudaFreeAsync(h->allocs.back(), h->stream));
+        CK(ctx_dev_free(h->ctx, h->allocs.back(), h->stream));
         h->allocs.pop_back();
     }
     if (iterations) *iterations = h->iterations;
