@@ -116,16 +116,16 @@ __global__ void __launch_bounds__(128, 7) k_brestrict(const BRec* __restrict__ r
 }
 
 template <int ROWS, int NT>
-__global__ void __launch_bounds__(NT, 1) k_bcoarsest(const BRec* __restrict__ recs, const int* __restrict__ list,
+__global__ void __launch_bounds__(CG_THREADS, 1) k_bcoarsest(const BRec* __restrict__ recs, const int* __restrict__ list,
                                                      const unsigned* __restrict__ active, int br, int outr) {
     griddep_wait();
     griddep_launch();
-    __shared__ float ps[NT * ROWS + 4];
+    extern __shared__ __align__(16) float cg_ps[];
     __shared__ __align__(16) float red[3][64];
     const int i = list[blockIdx.x];
     if (!active[i]) return;
     const BRec& R = recs[i];
-    coarsest_cg_body<ROWS, NT, false>(R.C, R.v[br], R.v[outr], ps, red);
+    coarsest_cg_body<ROWS, NT, false>(R.C, R.v[br], R.v[outr], cg_ps, red);
 }
 
 __global__ void __launch_bounds__(128) k_bdot_rho(const BRec* __restrict__ recs, const int2* __restrict__ map,
@@ -303,9 +303,15 @@ struct BEnq {
     void coarsest(int d, int br, int outr, bool dot) {
         const std::array<uaamg_batch::Range, 3>& c = b->coarse[d];
         const unsigned* act = b->active;
-        if (c[0].count) launch(k_bcoarsest<2, 512>, (unsigned)c[0].count, 512, s, recs(d), b->lists + c[0].off, act, br, outr);
-        if (c[1].count) launch(k_bcoarsest<4, 512>, (unsigned)c[1].count, 512, s, recs(d), b->lists + c[1].off, act, br, outr);
-        if (c[2].count) launch(k_bcoarsest<4, 1024>, (unsigned)c[2].count, 1024, s, recs(d), b->lists + c[2].off, act, br, outr);
+        if (c[0].count)
+            launch_smem(k_bcoarsest<2, 512>, (unsigned)c[0].count, CG_THREADS, cg_smem_bytes<2, 512>(), s, recs(d),
+                        b->lists + c[0].off, act, br, outr);
+        if (c[1].count)
+            launch_smem(k_bcoarsest<4, 512>, (unsigned)c[1].count, CG_THREADS, cg_smem_bytes<4, 512>(), s, recs(d),
+                        b->lists + c[1].off, act, br, outr);
+        if (c[2].count)
+            launch_smem(k_bcoarsest<4, 1024>, (unsigned)c[2].count, CG_THREADS, cg_smem_bytes<4, 1024>(), s, recs(d),
+                        b->lists + c[2].off, act, br, outr);
         count += (c[0].count > 0) + (c[1].count > 0) + (c[2].count > 0);
         if (dot && d == 0 && b->dot1.count) {
             launch(k_bdot_rho, (unsigned)b->dot1.count, 128, s, recs(0), map(b->dot1), act);
@@ -529,6 +535,8 @@ static void bbuild_tables(uaamg_batch* b) {
             r.count = (int)lists.size() - r.off;
         }
     }
+    CK(cudaFuncSetAttribute(k_bcoarsest<4, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            cg_smem_bytes<4, 1024>()));
     // one device allocation: records, maps, lists, active flags, pointer
     // arrays, global counters, gathered states
     const size_t nrec = (size_t)b->depth * n;

@@ -444,7 +444,7 @@ struct uaamg_poisson {
     // the bottom of the W-cycle in one cluster launch (k_bottom): decided once
     // per handle; level lb = nlev - 2, P leaves per CTA, a cluster of bot_C
     int bot_state = -1;  // -1 undecided, 0 not used (or turned off by UAAMG_BOTTOM=0 at creation), 1 used
-    int bot_C = 0, bot_P = 0, bot_rows = 0;
+    int bot_C = 0, bot_P = 0, bot_cls = 0, bot_nl = 0;
     size_t bot_smem = 0;
 };
 
@@ -927,6 +927,9 @@ static void build_hierarchy(uaamg_poisson* h, const uaamg_leaf_grid* phi, const 
             CK(cudaMemsetAsync(cur, 0, bytes - table_bytes, s));
             for (int l = 1; l < nlev; ++l) carve_arrays(h->host[l], h->lv[l], cur);
             h->C.n = (int)nc;
+            if (coarsest_class(h->C.n) == 2)  // above the 48 KB a launch may ask for unasked
+                CK(cudaFuncSetAttribute(k_coarsest_cg<4, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        cg_smem_bytes<4, 1024>()));
             dslot = carve<int>(cur, nc);
             cdiag = carve<float>(cur, nc);
             cinvd = carve<float>(cur, nc);
@@ -1068,36 +1071,15 @@ static void enq_memset(void* p, int v, size_t n, cudaStream_t s) {
 }
 
 template <typename... KArgs, typename... Args>
-static void launch(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args) {
+static void launch_smem(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                        Args... args) {
     if (t_rec) {
-        rec_launch(kern, dim3(grid), dim3(block), 0, g_use_pdl ? 1 : 0, args...);
+        rec_launch(kern, dim3(grid), dim3(block), smem, g_use_pdl ? 1 : 0, args...);
         return;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = g_use_pdl ? 1 : 0;
-    CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
-}
-
-// Launch of a pipelined staged kernel (staged_pipe.cuh) over nl leaves:
-// PIPE_CTAS CTAs, at most one per leaf.
-template <typename... KArgs, typename... Args>
-static void launch_pipe(void (*kern)(KArgs...), int nl, size_t smem, cudaStream_t s, Args... args) {
-    const int g = std::min(nl, PIPE_CTAS);
-    if (t_rec) {
-        rec_launch(kern, dim3((unsigned)g), dim3(128), smem, g_use_pdl ? 1 : 0, args...);
-        return;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)g);
-    cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -1106,6 +1088,67 @@ static void launch_pipe(void (*kern)(KArgs...), int nl, size_t smem, cudaStream_
     cfg.attrs = at;
     cfg.numAttrs = g_use_pdl ? 1 : 0;
     CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+}
+template <typename... KArgs, typename... Args>
+static void launch(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args) {
+    launch_smem(kern, grid, block, 0, s, args...);
+}
+
+// Launch of one thread-block cluster of C CTAs.
+template <typename... KArgs, typename... Args>
+static void launch_cluster(void (*kern)(KArgs...), int C, unsigned block, size_t smem, cudaStream_t s, Args... args) {
+    if (t_rec) {
+        rec_launch(kern, dim3((unsigned)C), dim3(block), smem, (g_use_pdl ? 2000 : 1000) + C, args...);
+        return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)C);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = g_use_pdl ? 2 : 1;
+    CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+}
+// Allows a kernel clusters above the portable size and `max_dynamic` bytes of
+// shared memory (the most any handle may use, so that no handle's setting
+// limits another's launches); whether the device can run a cluster of C CTAs
+// with `smem` bytes each.
+template <typename... KArgs>
+static bool cluster_fits(void (*kern)(KArgs...), int C, unsigned block, size_t smem, int max_dynamic) {
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic));
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)C);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n >= 1;
+}
+
+// Launch of a pipelined staged kernel (staged_pipe.cuh) over nl leaves:
+// PIPE_CTAS CTAs, at most one per leaf.
+template <typename... KArgs, typename... Args>
+static void launch_pipe(void (*kern)(KArgs...), int nl, size_t smem, cudaStream_t s, Args... args) {
+    launch_smem(kern, (unsigned)std::min(nl, PIPE_CTAS), 128, smem, s, args...);
 }
 
 // Optional per-kernel timing (diagnostics): a CUDA event pair around every launch.
@@ -1147,6 +1190,13 @@ template <> struct SrcName<SrcProlong> { static const char* get() { return "+pro
 static const char* mode_name(int m) {
     static const char* n[] = {"jacobi", "residual", "laplacian", "red_gs", "black_gs", "spai0"};
     return n[m];
+}
+
+// k_bottom by coarsest shape (coarsest_class) and leaves per thread
+static void (*bottom_kernel(int cls, int nl))(BottomArgs) {
+    if (cls == 0) return nl == 1 ? k_bottom<2, 512, 1> : k_bottom<2, 512, 2>;
+    if (cls == 1) return nl == 1 ? k_bottom<4, 512, 1> : k_bottom<4, 512, 2>;
+    return nl == 1 ? k_bottom<4, 1024, 1> : k_bottom<4, 1024, 2>;
 }
 
 struct Enq {
@@ -1251,29 +1301,7 @@ struct Enq {
         A.P = h->bot_P;
         A.w[0] = w[0]; A.w[1] = w[1]; A.w[2] = w[2];
         if (prof) pb("L" + std::to_string(lb) + " bottom (2 visits + coarsest)");
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)h->bot_C);
-        cfg.blockDim = dim3(BOT_THREADS);
-        cfg.dynamicSmemBytes = h->bot_smem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)h->bot_C;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = g_use_pdl ? 2 : 1;
-        if (t_rec) {
-            const int attrs = (int)cfg.numAttrs * 1000 + h->bot_C;  // the cluster shape
-            if (h->bot_rows == 2) rec_launch(k_bottom<2>, cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes, attrs, A);
-            else rec_launch(k_bottom<4>, cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes, attrs, A);
-        } else if (h->bot_rows == 2) {
-            CK(cudaLaunchKernelEx(&cfg, k_bottom<2>, A));
-        } else {
-            CK(cudaLaunchKernelEx(&cfg, k_bottom<4>, A));
-        }
+        launch_cluster(bottom_kernel(h->bot_cls, h->bot_nl), h->bot_C, BOT_THREADS, h->bot_smem, s, A);
         pe();
         count++;
     }
@@ -1281,9 +1309,11 @@ struct Enq {
         if (h->C.n == 0) return;
         pb("coarsest cg");
         switch (coarsest_class(h->C.n)) {
-            case 0: launch(k_coarsest_cg<2, 512>, 1, 512, s, h->C, rhs, out); break;
-            case 1: launch(k_coarsest_cg<4, 512>, 1, 512, s, h->C, rhs, out); break;
-            default: launch(k_coarsest_cg<4, 1024>, 1, 1024, s, h->C, rhs, out); break;
+            case 0: launch_smem(k_coarsest_cg<2, 512>, 1, CG_THREADS, cg_smem_bytes<2, 512>(), s, h->C, rhs, out); break;
+            case 1: launch_smem(k_coarsest_cg<4, 512>, 1, CG_THREADS, cg_smem_bytes<4, 512>(), s, h->C, rhs, out); break;
+            default:
+                launch_smem(k_coarsest_cg<4, 1024>, 1, CG_THREADS, cg_smem_bytes<4, 1024>(), s, h->C, rhs, out);
+                break;
         }
         pe();
         count++;
@@ -1292,33 +1322,10 @@ struct Enq {
 
 // Whether the two visits of level nlev - 2 (with the coarsest solves) run as
 // one k_bottom cluster launch: Jacobi-family smoothers, at least three levels,
-// a coarsest system the 256-thread CG shape takes (at most 2048 DOF), and a
-// cluster of at most 16 CTAs whose shared memory holds level nlev - 2 and
-// that the device can schedule.  The shape is decided once per handle.
+// at most BOT_MAX_NL leaves per thread in a cluster of 15 leaf CTAs (120
+// leaves), a coarsest level CTA 0 can hold, and a cluster the device can
+// schedule.  The shape is decided once per handle.
 static bool g_use_bottom = true;
-template <int R>
-static int bottom_clusters(int C, size_t smem, int max_dynamic) {
-    // the largest size any handle may use, so that no handle's setting limits another's launches
-    CK(cudaFuncSetAttribute(k_bottom<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic));
-    CK(cudaFuncSetAttribute(k_bottom<R>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)C);
-    cfg.blockDim = dim3(BOT_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_bottom<R>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return n;
-}
 static bool use_bottom(uaamg_poisson* h) {
     if (h->smoother != UAAMG_SMOOTHER_SCHEDULED_RELAXED_JACOBI && h->smoother != UAAMG_SMOOTHER_WEIGHTED_JACOBI)
         return false;
@@ -1327,20 +1334,22 @@ static bool use_bottom(uaamg_poisson* h) {
     if (h->nlev < 3) return false;
     const int lb = h->nlev - 2;
     const int nl = h->lv[lb].L.nl, nlc = h->lv[lb + 1].L.nl;
-    if (nl <= 0 || nlc <= 0 || h->C.n <= 0 || coarsest_class(h->C.n) > 1) return false;
-    const int P = (nl + BOT_MAX_CLUSTER - 1) / BOT_MAX_CLUSTER;
-    const int C = (nl + P - 1) / P;
-    const int rows = coarsest_class(h->C.n) == 0 ? 2 : 4;
-    const size_t smem = bottom_smem_bytes(P, nlc, rows);
+    if (nl <= 0 || nlc <= 0 || h->C.n <= 0 || h->C.n > CG_MAX_DOF) return false;
+    const int P = (nl + BOT_MAX_CLUSTER - 2) / (BOT_MAX_CLUSTER - 1);
+    if (P > BOT_GROUPS * BOT_MAX_NL) return false;
+    const int C = 1 + (nl + P - 1) / P;
+    const int cls = coarsest_class(h->C.n), per_thread = (P + BOT_GROUPS - 1) / BOT_GROUPS;
+    const size_t smem = cls == 0 ? bottom_smem_bytes<2, 512>(P, nlc)
+                                 : (cls == 1 ? bottom_smem_bytes<4, 512>(P, nlc) : bottom_smem_bytes<4, 1024>(P, nlc));
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->ctx->device));
     const int max_dynamic = optin - 1024;  // above the kernel's static shared memory
     if (smem > (size_t)max_dynamic) return false;
-    if ((rows == 2 ? bottom_clusters<2>(C, smem, max_dynamic) : bottom_clusters<4>(C, smem, max_dynamic)) < 1)
-        return false;
+    if (!cluster_fits(bottom_kernel(cls, per_thread), C, BOT_THREADS, smem, max_dynamic)) return false;
     h->bot_C = C;
     h->bot_P = P;
-    h->bot_rows = rows;
+    h->bot_cls = cls;
+    h->bot_nl = per_thread;
     h->bot_smem = smem;
     h->bot_state = 1;
     return true;

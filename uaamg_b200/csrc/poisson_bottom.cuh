@@ -5,16 +5,28 @@
 // level above it, and each visit is seven smoothing / transfer passes over a
 // few dozen leaves plus the coarsest CG: fourteen small launches that are
 // bound by launch latency, not by their bytes.  k_bottom runs both visits in
-// one launch of one thread-block cluster.  Level lb and the coarsest level
-// stay resident in the cluster's shared memory for the whole launch: every
-// leaf of level lb, with its vectors and coefficients, lives in the shared
-// memory of one CTA (leaf i in CTA i / P, slot i % P), the coarsest level's
-// vectors in CTA 0.  A stencil reads a neighbour leaf that another CTA holds
-// through distributed shared memory; passes are separated by cluster
-// barriers.  The per-voxel arithmetic is that of the unfused kernels
-// (sweep_value_s, restrict_leaf, k_materialize with SrcFirstJacobi /
-// SrcProlong, coarsest_cg_body with the same rows-per-thread shape), so the
-// results are bit-identical to the launch sequence it replaces.
+// one launch of one thread-block cluster.  CTA 0 holds the coarsest level and
+// does its CG; the other CTAs hold level lb, P leaves each (leaf i in CTA
+// 1 + i / P, slot i % P), a thread four voxels of NL leaves.  What another
+// thread reads (the two smoothing vectors) lives in shared memory, everything
+// else (rhs, coefficients, the thread's own values, the addresses of its
+// neighbours' values) in registers for the whole launch.
+//
+// Measured at 128^3 (40 leaves, 1,916 DOF below them; events around the
+// launch): 40.3 us, 47.7 us when the leaves' pointers were read and tested in
+// every pass and CTA 0 held leaves too.
+// What bounds a pass is one chain: neighbour loads (distributed shared memory
+// across CTAs), the stencil's arithmetic, the store, the cluster barrier.  The
+// loads are unconditional (an absent neighbour's address is a zero slot), so
+// they are in flight together; with the leaf's pointers read and tested per
+// pass they queued one after another.  The CG is a CTA of its own because the
+// registers of its matrix rows and of a leaf's stencil do not fit one thread
+// together, and so the rows are loaded once for both visits.
+//
+// The per-voxel arithmetic is that of the unfused kernels (sweep_value_s,
+// restrict_leaf, k_materialize with SrcFirstJacobi / SrcProlong,
+// cg_rows_solve), so the results are bit-identical to the launch sequence it
+// replaces.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -24,20 +36,10 @@ namespace uaamg {
 
 namespace cgx = cooperative_groups;
 
-constexpr int BOT_THREADS = 512;     // four 128-thread leaf groups; the coarsest CG's block shape
-constexpr int BOT_MAX_CLUSTER = 16;  // non-portable cluster size limit
-constexpr int BOT_NT = 512;          // threads of the coarsest CG (coarsest_class 0 and 1)
-
-// One leaf of level lb in shared memory.
-struct __align__(16) SLeaf {
-    float x[UAAMG_LEAF], b[UAAMG_LEAF], t[UAAMG_LEAF];
-    float dg[UAAMG_LEAF], iv[UAAMG_LEAF], cx[UAAMG_LEAF], cy[UAAMG_LEAF], cz[UAAMG_LEAF];
-    float fxp[64], fyp[64], fzp[64];  // c_x of the +x neighbour's x = 0 face [y][z], c_y of +y's [x][z], c_z of +z's [x][y]
-    uint64_t mask[8];
-    const SLeaf* nb[6];               // neighbour leaves (-x,+x,-y,+y,-z,+z) as cluster-shared addresses, or null
-    int par, oct;                     // parent leaf on the coarsest level, octant in it
-};
-constexpr int SLEAF_X = 0, SLEAF_T = 2 * UAAMG_LEAF;  // float offsets of the x and t arrays
+constexpr int BOT_THREADS = CG_THREADS;  // the coarsest CG's block; four 128-thread leaf groups
+constexpr int BOT_GROUPS = BOT_THREADS / 128;
+constexpr int BOT_MAX_CLUSTER = 16;      // non-portable cluster size limit
+constexpr int BOT_MAX_NL = 2;            // leaves per thread: more do not fit its registers
 
 struct BottomArgs {
     DLevel L;              // level lb
@@ -49,8 +51,6 @@ struct BottomArgs {
     float w[3];            // pre-smoothing weights (post-smoothing uses them reversed)
 };
 
-__device__ __forceinline__ float4 lds4(const float* p, int i) { return reinterpret_cast<const float4*>(p)[i]; }
-__device__ __forceinline__ void sts4(float* p, int i, float4 v) { reinterpret_cast<float4*>(p)[i] = v; }
 __device__ __forceinline__ float4 mask_out(float4 v, unsigned m) {
     if (!(m & 1)) v.x = 0.f;
     if (!(m & 2)) v.y = 0.f;
@@ -58,53 +58,121 @@ __device__ __forceinline__ float4 mask_out(float4 v, unsigned m) {
     if (!(m & 8)) v.w = 0.f;
     return v;
 }
-__device__ __forceinline__ unsigned smask4(const SLeaf* s, int t) {
-    return (unsigned)((s->mask[t >> 4] >> ((t & 15) * 4)) & 0xFull);
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// loads and stores at shared-memory addresses of the cluster (this CTA's own included)
+__device__ __forceinline__ unsigned dsm_map(const void* p, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float4 dsm_ld4(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 dsm_ld2(unsigned a) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float dsm_ld1(unsigned a) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void dsm_st1(unsigned a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 
-// stencil_dyn over shared-memory leaves: the 6-neighbour sum of the float4 of
-// thread t, source array at float offset `so` of every leaf
-__device__ __forceinline__ void bot_stencil(const SLeaf* me, int so, int t, float4& xc, float4& off) {
-    const int X = t >> 4, Y = (t >> 1) & 7, zh = t & 1;
-    const float* src = reinterpret_cast<const float*>(me) + so;
-    xc = lds4(src, t);
-    float4 xp, xm, yp, ym;
-    if (X < 7) xp = lds4(src, t + 16);
-    else xp = me->nb[1] ? lds4(reinterpret_cast<const float*>(me->nb[1]) + so, t - 112) : f4zero();
-    if (X > 0) xm = lds4(src, t - 16);
-    else xm = me->nb[0] ? lds4(reinterpret_cast<const float*>(me->nb[0]) + so, t + 112) : f4zero();
-    if (Y < 7) yp = lds4(src, t + 2);
-    else yp = me->nb[3] ? lds4(reinterpret_cast<const float*>(me->nb[3]) + so, t - 14) : f4zero();
-    if (Y > 0) ym = lds4(src, t - 2);
-    else ym = me->nb[2] ? lds4(reinterpret_cast<const float*>(me->nb[2]) + so, t + 14) : f4zero();
-    const float4 cxp = X < 7 ? lds4(me->cx, t + 16) : lds4(me->fxp, Y * 2 + zh);
-    const float4 cyp = Y < 7 ? lds4(me->cy, t + 2) : lds4(me->fyp, X * 2 + zh);
-    const float4 cxm = lds4(me->cx, t), cym = lds4(me->cy, t), czo = lds4(me->cz, t);
+// Shared memory of a leaf CTA: per leaf slot the vectors x and t, then a slot
+// of zeros.  Offsets in bytes.
+constexpr unsigned BOT_X = 0, BOT_T = UAAMG_LEAF * 4, BOT_SLOT = 2 * UAAMG_LEAF * 4;
+
+// One thread's part of one leaf of level lb.
+struct BotLeaf {
+    bool on;                                     // the leaf exists
+    int leaf;
+    unsigned m;                                  // DOF bits
+    unsigned own, xp, xm, yp, ym, zn;            // addresses of the thread's float4, its neighbours', the +-z neighbour
+    unsigned cr, cp, cm;                         // coarse rhs word it restricts to, coarse pair it prolongs, child bits
+    float4 b, dg, iv, cxp, cxm, cyp, cym, czo;   // rhs and coefficients (sweep_static)
+    float czp3;
+    float4 v;                                    // the thread's values of the vector written last
+};
+
+// the leaf's static data, before the wait for the previous kernel
+__device__ __forceinline__ void bot_load(const BottomArgs& A, BotLeaf& B, unsigned char* sm, int leaf, int slot, int t,
+                                         const float* bc, const float* xc) {
+    const DLevel& L = A.L;
+    const int P = A.P, X = t >> 4, Y = (t >> 1) & 7, zh = t & 1;
+    const unsigned zero = smem_u32(sm) + (unsigned)P * BOT_SLOT;
+    B.leaf = leaf;
+    B.on = slot < P && leaf < L.nl;
+    B.m = 0;
+    if (!B.on) return;
+    PStatic S;
+    stencil_static(L, leaf, t, S);
+    B.cxp = S.cxp; B.cxm = S.cxm; B.cyp = S.cyp; B.cym = S.cym; B.czo = S.czo;
+    const float pcz = __shfl_xor_sync(FULLMASK, S.czo.x, 1);
+    B.czp3 = zh == 0 ? pcz : S.czp3;
+    B.dg = (S.fl & TRIM_DIAG) ? f4splat(L.def_diag) : ld4(L.diag, leaf, t);
+    B.iv = (S.fl & TRIM_DIAG) ? f4splat(L.def_invdiag) : ld4(L.invdiag, leaf, t);
+    B.m = mask4(L.mask, leaf, t);
+    B.own = smem_u32(sm) + (unsigned)slot * BOT_SLOT + 16u * t;
+    // a neighbour leaf's slot, as the cluster addresses it
+    auto at = [&](int n, int off) {
+        return n < 0 ? zero : dsm_map(sm + (size_t)(n % P) * BOT_SLOT, 1u + (unsigned)(n / P)) + 4u * off;
+    };
+    B.xp = X < 7 ? B.own + 16u * 16 : at(S.nxp, 4 * (t - 112));
+    B.xm = X > 0 ? B.own - 16u * 16 : at(S.nxm, 4 * (t + 112));
+    B.yp = Y < 7 ? B.own + 16u * 2 : at(S.nyp, 4 * (t - 14));
+    B.ym = Y > 0 ? B.own - 16u * 2 : at(S.nym, 4 * (t + 14));
+    B.zn = zh == 0 ? at(S.nzm, 4 * t + 7) : at(S.nzp, 4 * t - 4);
+    const int par = L.parent[leaf], o = L.octant[leaf];
+    const int cX = ((o >> 2) & 1) * 4, cY = ((o >> 1) & 1) * 4, cZ = (o & 1) * 4;
+    B.cp = dsm_map(xc + (size_t)par * UAAMG_LEAF + (cX + (X >> 1)) * 64 + (cY + (Y >> 1)) * 8 + cZ + 2 * zh, 0);
+    // t < 64: coarse voxel (i, j, k) of the octant, its eight fine voxels
+    const int i = (t >> 4) & 3, j = (t >> 2) & 3, k = t & 3;
+    B.cr = dsm_map(bc + (size_t)par * UAAMG_LEAF + ((cX + i) << 6) + ((cY + j) << 3) + cZ + k, 0);
+    B.cm = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int fo = ((2 * i + (q >> 2)) << 6) | ((2 * j + ((q >> 1) & 1)) << 3) | (2 * k + (q & 1));
+        B.cm |= (unsigned)((L.mask[(long long)leaf * 8 + (fo >> 6)] >> (fo & 63)) & 1ull) << q;
+    }
+}
+
+__device__ __forceinline__ void bot_store(const BotLeaf& B, unsigned dst) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(B.own + dst), "f"(B.v.x), "f"(B.v.y), "f"(B.v.z),
+                 "f"(B.v.w)
+                 : "memory");
+}
+
+// stencil_dyn: the 6-neighbour sum of the thread's float4 (B.v) over the vector at byte offset src
+__device__ __forceinline__ float4 bot_stencil(const BotLeaf& B, unsigned src, int zh) {
+    const float4 xp = dsm_ld4(B.xp + src), xm = dsm_ld4(B.xm + src);
+    const float4 yp = dsm_ld4(B.yp + src), ym = dsm_ld4(B.ym + src);
+    const float zn = dsm_ld1(B.zn + src);
+    const float4 xc = B.v;
     const float px = __shfl_xor_sync(FULLMASK, xc.x, 1);
     const float pw = __shfl_xor_sync(FULLMASK, xc.w, 1);
-    const float pcz = __shfl_xor_sync(FULLMASK, czo.x, 1);
-    const int base = 4 * t;
-    float zp3, zm0, czp3;
-    if (zh == 0) {
-        zp3 = px;
-        czp3 = pcz;
-        zm0 = me->nb[4] ? reinterpret_cast<const float*>(me->nb[4])[so + base + 7] : 0.f;
-    } else {
-        zm0 = pw;
-        zp3 = me->nb[5] ? reinterpret_cast<const float*>(me->nb[5])[so + base - 4] : 0.f;
-        czp3 = me->fzp[X * 8 + Y];
-    }
-    const float zp[4] = {xc.y, xc.z, xc.w, zp3};
-    const float zm[4] = {zm0, xc.x, xc.y, xc.z};
-    const float czp[4] = {czo.y, czo.z, czo.w, czp3};
+    const float zp[4] = {xc.y, xc.z, xc.w, zh == 0 ? px : zn};
+    const float zm[4] = {zh == 0 ? zn : pw, xc.x, xc.y, xc.z};
+    const float czp[4] = {B.czo.y, B.czo.z, B.czo.w, B.czp3};
+    float4 off;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        float f1 = __fmul_rn(f4get(xp, j), f4get(cxp, j));
-        float f2 = __fmul_rn(f4get(xm, j), f4get(cxm, j));
-        float f3 = __fmul_rn(f4get(yp, j), f4get(cyp, j));
-        float f4 = __fmul_rn(f4get(ym, j), f4get(cym, j));
+        float f1 = __fmul_rn(f4get(xp, j), f4get(B.cxp, j));
+        float f2 = __fmul_rn(f4get(xm, j), f4get(B.cxm, j));
+        float f3 = __fmul_rn(f4get(yp, j), f4get(B.cyp, j));
+        float f4 = __fmul_rn(f4get(ym, j), f4get(B.cym, j));
         float f5 = __fmul_rn(zp[j], czp[j]);
-        float f6 = __fmul_rn(zm[j], f4get(czo, j));
+        float f6 = __fmul_rn(zm[j], f4get(B.czo, j));
         f1 = __fadd_rn(f1, f2);
         f3 = __fadd_rn(f3, f4);
         f5 = __fadd_rn(f5, f6);
@@ -112,190 +180,133 @@ __device__ __forceinline__ void bot_stencil(const SLeaf* me, int so, int t, floa
         f1 = __fadd_rn(f1, f5);
         f4set(off, j, f1);
     }
+    return off;
 }
-
-// weighted Jacobi (sweep_value_s<M_JACOBI>): out = x + w invdiag (b - A x)
-__device__ __forceinline__ void bot_jacobi(SLeaf* me, int so, int dst, int t, float w) {
-    float4 xc, off;
-    bot_stencil(me, so, t, xc, off);
-    const float4 bb = lds4(me->b, t), dg = lds4(me->dg, t), iv = lds4(me->iv, t);
+// weighted Jacobi (sweep_value_s<M_JACOBI>): v = x + w invdiag (b - A x)
+__device__ __forceinline__ void bot_jacobi(BotLeaf& B, unsigned src, float w, int zh) {
+    const float4 off = bot_stencil(B, src, zh);
     float4 res;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        float r = __fsub_rn(f4get(bb, j), __fmaf_rn(f4get(xc, j), f4get(dg, j), f4get(off, j)));
-        r = __fmul_rn(r, f4get(iv, j));
-        f4set(res, j, __fmaf_rn(w, r, f4get(xc, j)));
+        float r = __fsub_rn(f4get(B.b, j), __fmaf_rn(f4get(B.v, j), f4get(B.dg, j), f4get(off, j)));
+        r = __fmul_rn(r, f4get(B.iv, j));
+        f4set(res, j, __fmaf_rn(w, r, f4get(B.v, j)));
     }
-    sts4(reinterpret_cast<float*>(me) + dst, t, mask_out(res, smask4(me, t)));
+    B.v = mask_out(res, B.m);
 }
-
-// residual of T restricted into the coarsest rhs held by CTA 0 (restrict_leaf<true>)
-__device__ __forceinline__ void bot_restrict(SLeaf* me, int t, float* rs, float* bc0, int group) {
-    float4 xc, off;
-    bot_stencil(me, SLEAF_T, t, xc, off);
-    const float4 bb = lds4(me->b, t), dg = lds4(me->dg, t);
+// residual of t restricted into the coarsest rhs of CTA 0 (restrict_leaf<true>);
+// the leaf's x, which nobody reads in this pass, carries the residual.  Called by
+// the whole 128-thread group.
+__device__ __forceinline__ void bot_restrict(const BotLeaf& B, int t, int group) {
+    const float4 off = bot_stencil(B, BOT_T, t & 1);
     float4 res;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        f4set(res, j, __fsub_rn(f4get(bb, j), __fmaf_rn(f4get(xc, j), f4get(dg, j), f4get(off, j))));
-    sts4(rs, t, mask_out(res, smask4(me, t)));
+        f4set(res, j, __fsub_rn(f4get(B.b, j), __fmaf_rn(f4get(B.v, j), f4get(B.dg, j), f4get(off, j))));
+    res = mask_out(res, B.m);
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(B.own + BOT_X), "f"(res.x), "f"(res.y), "f"(res.z),
+                 "f"(res.w)
+                 : "memory");
     asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
     if (t < 64) {
         const int i = t >> 4, j = (t >> 2) & 3, k = t & 3;
+        const unsigned rs = B.own - 16u * t + 4u * (((2 * i) << 6) | ((2 * j) << 3) | (2 * k));
         float s = 0.f;
 #pragma unroll
-        for (int ii = 0; ii < 2; ++ii)
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-                    int fo = ((2 * i + ii) << 6) | ((2 * j + jj) << 3) | (2 * k + kk);
-                    if ((me->mask[fo >> 6] >> (fo & 63)) & 1ull) s = __fadd_rn(s, rs[fo]);
-                }
-        const int o = me->oct;
-        const int coff = ((((o >> 2) & 1) * 4 + i) << 6) | ((((o >> 1) & 1) * 4 + j) << 3) | ((o & 1) * 4 + k);
-        bc0[(long long)me->par * UAAMG_LEAF + coff] = __fmul_rn(s, 0.125f);
+        for (int q = 0; q < 4; ++q) {
+            const float2 u = dsm_ld2(rs + 4u * (64 * (q >> 1) + 8 * (q & 1)));
+            if ((B.cm >> (2 * q)) & 1) s = __fadd_rn(s, u.x);
+            if ((B.cm >> (2 * q + 1)) & 1) s = __fadd_rn(s, u.y);
+        }
+        dsm_st1(B.cr, __fmul_rn(s, 0.125f));
     }
-    asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+}
+// v += x_c(parent voxel) on the DOF (SrcProlong with alpha 1)
+__device__ __forceinline__ void bot_prolong(BotLeaf& B) {
+    const float2 c = dsm_ld2(B.cp);
+    const float c0 = __fmul_rn(1.0f, c.x), c1 = __fmul_rn(1.0f, c.y);
+    if (B.m & 1) B.v.x = __fadd_rn(B.v.x, c0);
+    if (B.m & 2) B.v.y = __fadd_rn(B.v.y, c0);
+    if (B.m & 4) B.v.z = __fadd_rn(B.v.z, c1);
+    if (B.m & 8) B.v.w = __fadd_rn(B.v.w, c1);
+    B.v = mask_out(B.v, B.m);
 }
 
-// T = w invdiag b (the first sweep from zero, SrcFirstJacobi, materialised)
-__device__ __forceinline__ void bot_first(SLeaf* me, int t, float w) {
-    const float4 bb = lds4(me->b, t), iv = lds4(me->iv, t);
-    const float4 v = make_float4(__fmul_rn(w, __fmul_rn(iv.x, bb.x)), __fmul_rn(w, __fmul_rn(iv.y, bb.y)),
-                                 __fmul_rn(w, __fmul_rn(iv.z, bb.z)), __fmul_rn(w, __fmul_rn(iv.w, bb.w)));
-    sts4(me->t, t, mask_out(v, smask4(me, t)));
+// dynamic shared memory of every CTA: CTA 0's coarse vectors and CG storage, or the leaf slots
+template <int ROWS, int NT>
+constexpr size_t bottom_smem_bytes(int P, int nlc) {
+    const size_t cg = (size_t)CgShape<ROWS, NT>::SMEM_FLOATS * 4 + (size_t)nlc * UAAMG_LEAF * 4 * 2;
+    const size_t leaves = (size_t)(P + 1) * BOT_SLOT;
+    return cg > leaves ? cg : leaves;
 }
 
-// T += x_c(parent voxel) on the DOF (SrcProlong with alpha 1, materialised)
-__device__ __forceinline__ void bot_prolong(SLeaf* me, int t, const float* xc0) {
-    float4 v = lds4(me->t, t);
-    const unsigned m = smask4(me, t);
-    if (m) {
-        const int o = me->oct;
-        const int X = t >> 4, Y = (t >> 1) & 7, zh = t & 1;
-        const int coff =
-            (((o >> 2) & 1) * 4 + (X >> 1)) * 64 + (((o >> 1) & 1) * 4 + (Y >> 1)) * 8 + (o & 1) * 4 + 2 * zh;
-        const float* cp = xc0 + (long long)me->par * UAAMG_LEAF + coff;
-        const float c0 = __fmul_rn(1.0f, cp[0]), c1 = __fmul_rn(1.0f, cp[1]);
-        if (m & 1) v.x = __fadd_rn(v.x, c0);
-        if (m & 2) v.y = __fadd_rn(v.y, c0);
-        if (m & 4) v.z = __fadd_rn(v.z, c1);
-        if (m & 8) v.w = __fadd_rn(v.w, c1);
-    }
-    sts4(me->t, t, mask_out(v, m));
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Dynamic shared memory of one CTA: P leaves, then (used by CTA 0 only) the
-// coarsest level's lhs and rhs, the CG's vector, one restriction scratch per
-// leaf group.
-__host__ __device__ inline size_t bottom_smem_bytes(int P, int nlc, int rows) {
-    return (size_t)P * sizeof(SLeaf) + (size_t)nlc * UAAMG_LEAF * 4 * 2 + (size_t)(BOT_NT * rows + 4) * 4 +
-           (size_t)(BOT_THREADS / 128) * UAAMG_LEAF * 4;
-}
-
-template <int ROWS>
+// Barriers of the cluster, the same for every CTA: start; per visit the two
+// (first visit; else three) sweeps, the restriction, the CG, the prolongation
+// and three sweeps.
+template <int ROWS, int NT, int NL>
 __global__ void __launch_bounds__(BOT_THREADS, 1) k_bottom(BottomArgs A) {
     extern __shared__ __align__(16) unsigned char bsm[];
     __shared__ __align__(16) float red[3][64];
-    cgx::cluster_group cl = cgx::this_cluster();
-    const unsigned rank = cl.block_rank();
-    const int group = threadIdx.x >> 7, t = threadIdx.x & 127;
-    constexpr int NG = BOT_THREADS / 128;
-    const int P = A.P;
-    SLeaf* sl = reinterpret_cast<SLeaf*>(bsm);
-    float* xc0 = reinterpret_cast<float*>(bsm + (size_t)P * sizeof(SLeaf));  // coarsest lhs (CTA 0)
-    float* bc0 = xc0 + (size_t)A.nlc * UAAMG_LEAF;                            // coarsest rhs (CTA 0)
-    float* ps = bc0 + (size_t)A.nlc * UAAMG_LEAF;
-    float* rs = ps + BOT_NT * ROWS + 4 + group * UAAMG_LEAF;
-    // the coarsest vectors of CTA 0 as every CTA addresses them
-    float* xc0c = cl.map_shared_rank(xc0, 0);
-    float* bc0c = cl.map_shared_rank(bc0, 0);
-    const DLevel& L = A.L;
-    const int nl = L.nl;
-
-    // ---- static data (does not change during a solve): before the wait
-    for (int j = group; j < P; j += NG) {
-        SLeaf* me = sl + j;
-        const int leaf = (int)rank * P + j;
-        if (leaf >= nl) continue;
-        const unsigned fl = L.flags[leaf];
-        const float4 dfv = f4splat(L.def_face);
-        sts4(me->dg, t, (fl & TRIM_DIAG) ? f4splat(L.def_diag) : ld4(L.diag, leaf, t));
-        sts4(me->iv, t, (fl & TRIM_DIAG) ? f4splat(L.def_invdiag) : ld4(L.invdiag, leaf, t));
-        sts4(me->cx, t, (fl & TRIM_X) ? dfv : ld4(L.cx, leaf, t));
-        sts4(me->cy, t, (fl & TRIM_Y) ? dfv : ld4(L.cy, leaf, t));
-        sts4(me->cz, t, (fl & TRIM_Z) ? dfv : ld4(L.cz, leaf, t));
-        const int* nb = L.nbr + (long long)leaf * 6;
-        if (t < 64) {
-            // + faces: (y,z) / (x,z) / (x,y) = (t >> 3, t & 7)
-            const int a = t >> 3, c = t & 7;
-            const int n1 = nb[1], n3 = nb[3], n5 = nb[5];
-            me->fxp[t] = n1 >= 0 ? ((L.flags[n1] & TRIM_X) ? L.def_face : L.cx[(long long)n1 * UAAMG_LEAF + a * 8 + c])
-                                 : L.def_face;
-            me->fyp[t] = n3 >= 0 ? ((L.flags[n3] & TRIM_Y) ? L.def_face : L.cy[(long long)n3 * UAAMG_LEAF + a * 64 + c])
-                                 : L.def_face;
-            me->fzp[t] = n5 >= 0 ? ((L.flags[n5] & TRIM_Z) ? L.def_face : L.cz[(long long)n5 * UAAMG_LEAF + a * 64 + c * 8])
-                                 : L.def_face;
-        } else if (t < 72) {
-            me->mask[t - 64] = L.mask[(long long)leaf * 8 + (t - 64)];
-        } else if (t < 78) {
-            const int n = nb[t - 72];
-            me->nb[t - 72] = n >= 0 ? cl.map_shared_rank(sl + (n % P), (unsigned)(n / P)) : nullptr;
-        } else if (t == 78) {
-            me->par = L.parent[leaf];
-            me->oct = L.octant[leaf];
+    const unsigned rank = cgx::this_cluster().block_rank();
+    // CTA 0's layout: the CG's storage, the coarsest lhs and rhs
+    float* ps = reinterpret_cast<float*>(bsm);
+    float* xc = ps + CgShape<ROWS, NT>::SMEM_FLOATS;
+    float* bc = xc + (size_t)A.nlc * UAAMG_LEAF;
+    if (rank == 0) {
+        CgRows<ROWS, NT> M;
+        cg_rows_load<ROWS, NT>(A.C, M, ps);
+        griddep_wait();
+        griddep_launch();
+        cluster_sync_all();
+#pragma unroll 1
+        for (int visit = 0; visit < 2; ++visit) {
+#pragma unroll 1
+            for (int i = 0; i < 3 + visit; ++i) cluster_sync_all();
+            cg_rows_solve<ROWS, NT>(A.C, M, bc, xc, ps, red);
+#pragma unroll 1
+            for (int i = 0; i < 5; ++i) cluster_sync_all();
         }
+        return;
     }
+    const int group = threadIdx.x >> 7, t = threadIdx.x & 127, zh = t & 1;
+    BotLeaf B[NL];
+#pragma unroll
+    for (int q = 0; q < NL; ++q) {
+        const int slot = group + q * BOT_GROUPS;
+        bot_load(A, B[q], bsm, ((int)rank - 1) * A.P + slot, slot, t, bc, xc);
+    }
+    if (threadIdx.x < BOT_SLOT / 16) reinterpret_cast<float4*>(bsm + (size_t)A.P * BOT_SLOT)[threadIdx.x] = f4zero();
     griddep_wait();
     griddep_launch();
-    for (int j = group; j < P; j += NG) {
-        const int leaf = (int)rank * P + j;
-        if (leaf < nl) sts4(sl[j].b, t, ld4(A.rhs, leaf, t));
-    }
-    cluster_sync_all();  // every CTA has started and filled its leaves
-
     const float w0 = A.w[0], w1 = A.w[1], w2 = A.w[2];
-#define BOT_EACH(body)                                      \
-    for (int j = group; j < P; j += NG) {                   \
-        SLeaf* me = sl + j;                                 \
-        if ((int)rank * P + j < nl) { body; }               \
-    }                                                       \
+#define BOT_EACH(body)                 \
+    _Pragma("unroll")                  \
+    for (int q = 0; q < NL; ++q)       \
+        if (B[q].on) { body; }         \
     cluster_sync_all();
+    // rhs; t = first sweep from zero, w invdiag b.  The barrier: every CTA has started and filled its leaves
+    BOT_EACH(B[q].b = ld4(A.rhs, B[q].leaf, t);
+             B[q].v = mask_out(make_float4(__fmul_rn(w0, __fmul_rn(B[q].iv.x, B[q].b.x)),
+                                           __fmul_rn(w0, __fmul_rn(B[q].iv.y, B[q].b.y)),
+                                           __fmul_rn(w0, __fmul_rn(B[q].iv.z, B[q].b.z)),
+                                           __fmul_rn(w0, __fmul_rn(B[q].iv.w, B[q].b.w))), B[q].m);
+             bot_store(B[q], BOT_T));
+#pragma unroll 1
     for (int visit = 0; visit < 2; ++visit) {
-        // pre-smoothing, ends in T
-        if (visit == 0) {
-            BOT_EACH(bot_first(me, t, w0));                  // T = first sweep from zero
-            BOT_EACH(bot_jacobi(me, SLEAF_T, SLEAF_X, t, w1));  // x = J(T)
-            BOT_EACH(bot_jacobi(me, SLEAF_X, SLEAF_T, t, w2));  // T = J(x)
-        } else {
-            BOT_EACH(bot_jacobi(me, SLEAF_X, SLEAF_T, t, w0));
-            BOT_EACH(bot_jacobi(me, SLEAF_T, SLEAF_X, t, w1));
-            BOT_EACH(bot_jacobi(me, SLEAF_X, SLEAF_T, t, w2));
-        }
-        // residual of T restricted into the coarsest rhs
-        BOT_EACH(bot_restrict(me, t, rs, bc0c, group));
-        // coarsest solve (its second visit in the W-cycle re-solves the same system: skipped).  The rows
-        // are loaded from L2 for each solve: holding them in registers across the whole kernel measured
-        // three times slower (31 against 11 us per solve on the 1916-DOF level)
-        if (rank == 0) coarsest_cg_body<ROWS, BOT_NT, false>(A.C, bc0, xc0, ps, red);
-        cluster_sync_all();
-        // post-smoothing with reversed weights: T += P x_c, x = J(T), T = J(x), x = J(T)
-        BOT_EACH(bot_prolong(me, t, xc0c));
-        BOT_EACH(bot_jacobi(me, SLEAF_T, SLEAF_X, t, w2));
-        BOT_EACH(bot_jacobi(me, SLEAF_X, SLEAF_T, t, w1));
-        BOT_EACH(bot_jacobi(me, SLEAF_T, SLEAF_X, t, w0));
+        // pre-smoothing, ends in t
+        if (visit) { BOT_EACH(bot_jacobi(B[q], BOT_X, w0, zh); bot_store(B[q], BOT_T)); }
+        BOT_EACH(bot_jacobi(B[q], BOT_T, w1, zh); bot_store(B[q], BOT_X));
+        BOT_EACH(bot_jacobi(B[q], BOT_X, w2, zh); bot_store(B[q], BOT_T));
+        BOT_EACH(bot_restrict(B[q], t, group));
+        cluster_sync_all();  // the coarsest solve (its second visit in the W-cycle re-solves the same system: skipped)
+        // post-smoothing with reversed weights: t += P x_c, x = J(t), t = J(x), x = J(t)
+        BOT_EACH(bot_prolong(B[q]); bot_store(B[q], BOT_T));
+        BOT_EACH(bot_jacobi(B[q], BOT_T, w2, zh); bot_store(B[q], BOT_X));
+        BOT_EACH(bot_jacobi(B[q], BOT_X, w1, zh); bot_store(B[q], BOT_T));
+        // the last barrier also keeps this CTA's shared memory until nobody reads it
+        BOT_EACH(bot_jacobi(B[q], BOT_T, w0, zh); if (visit) st4(A.lhs, B[q].leaf, t, B[q].v); else bot_store(B[q], BOT_X));
     }
 #undef BOT_EACH
-    for (int j = group; j < P; j += NG) {
-        const int leaf = (int)rank * P + j;
-        if (leaf < nl) st4(A.lhs, leaf, t, lds4(sl[j].x, t));
-    }
-    // (the last pass ended with a cluster barrier, so no CTA still reads another's shared memory)
 }
 
 }  // namespace uaamg

@@ -1348,13 +1348,31 @@ struct DCoarsest {
     const float* val;      // [n][6]
 };
 
-// Thread-block shapes of the coarsest CG, by system size (rows per thread,
-// threads): 512 threads with 2 or 4 rows each up to 2048 DOF, 1024 threads
-// with 4 rows above; the rows' entries stay in registers.  The batched solve
-// and the cluster bottom-cycle kernel use the same shape for the same size, so
-// their results match the single solve bit for bit.
+// Shapes of the coarsest CG by system size: row i belongs to lane i mod NT, a
+// lane's rows are summed in a chain, lanes in warps of 32, the NT / 32 warp
+// sums in one tree.  512 lanes with 2 or 4 rows each up to 2048 DOF, 1024
+// lanes with 4 rows above.  The batched solve and the cluster bottom-cycle
+// kernel use the same shape for the same size, so their results match the
+// single solve bit for bit.
 #define CG_MAX_DOF 4096
 __host__ __device__ __forceinline__ int coarsest_class(int n) { return n <= 1024 ? 0 : (n <= 2048 ? 1 : 2); }
+
+// A block of CG_THREADS threads runs every shape; with 1024 lanes a thread is
+// lanes tid and tid + 512.  (1024 threads of 64 registers could not hold four
+// rows: they spilled, and the solve of 3,360 DOF took 37.5 us, 30.5 us now by
+// events around the launch.)
+constexpr int CG_THREADS = 512;
+template <int ROWS, int NT>
+struct CgShape {
+    static constexpr int V = NT / CG_THREADS;  // lanes per thread
+    static constexpr int R = ROWS * V;         // rows per thread
+    // With eight rows a thread's matrix entries fill its registers: 1/diag,
+    // diag and x then live in shared memory (each word used by its own thread
+    // only), and the columns are packed as two 16-bit byte offsets.
+    static constexpr bool LEAN = V > 1;
+    static constexpr int N = NT * ROWS;
+    static constexpr int SMEM_FLOATS = N + 4 + (LEAN ? 3 * N : 0);
+};
 
 // Block reductions in one barrier: warps reduce with shfl_down into lane 0,
 // lane 0 of each warp publishes its partial, and every thread then adds the
@@ -1382,57 +1400,88 @@ __device__ __forceinline__ float cg_tree_sum(const float* buf) {
         for (int q = 0; q + step < NW / 4; q += 2 * step) s[q] += s[q + step];
     return s[0];
 }
-template <int NT>
-__device__ __forceinline__ float cg_block_sum(float v, float* buf) {
+template <int V>
+__device__ __forceinline__ float cg_block_sum(const float* v, float* buf) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    v = cg_warp_partial(v);
-    if (lane == 0) buf[w] = v;
+    float a[V];
+#pragma unroll
+    for (int q = 0; q < V; ++q) a[q] = cg_warp_partial(v[q]);
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) buf[w + q * (CG_THREADS / 32)] = a[q];
+    }
     __syncthreads();
-    return cg_tree_sum<NT / 32>(buf);
+    return cg_tree_sum<V * CG_THREADS / 32>(buf);
 }
-template <int NT>
-__device__ __forceinline__ float2 cg_block_sum2(float a, float b, float* buf) {
+template <int V>
+__device__ __forceinline__ float2 cg_block_sum2(const float* va, const float* vb, float* buf) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float a[V], b[V];
+#pragma unroll
+    for (int q = 0; q < V; ++q) a[q] = va[q], b[q] = vb[q];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(FULLMASK, a, o);
-        b += __shfl_down_sync(FULLMASK, b, o);
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            a[q] += __shfl_down_sync(FULLMASK, a[q], o);
+            b[q] += __shfl_down_sync(FULLMASK, b[q], o);
+        }
     }
-    if (lane == 0) { buf[w] = a; buf[32 + w] = b; }
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            buf[w + q * (CG_THREADS / 32)] = a[q];
+            buf[32 + w + q * (CG_THREADS / 32)] = b[q];
+        }
+    }
     __syncthreads();
-    return make_float2(cg_tree_sum<NT / 32>(buf), cg_tree_sum<NT / 32>(buf + 32));
+    return make_float2(cg_tree_sum<V * CG_THREADS / 32>(buf), cg_tree_sum<V * CG_THREADS / 32>(buf + 32));
 }
 
-// ROWS rows per thread in a block of NT threads (row i = tid + k * NT); the
-// matrix rows stay in registers for the whole solve (CgRows), so a kernel that
+// A thread's matrix rows, in registers for the whole solve, so a kernel that
 // solves the same system twice loads them once.  Three barriers per CG
 // iteration.  (Publishing z and the old p with the second reduction, so that
 // each thread forms its neighbours' new p itself and one barrier goes, doubles
 // the shared-memory reads in flight and pushes the rows out of registers:
 // measured 1.6 times slower.)
-template <int ROWS>
-struct CgRows {
-    float dg[ROWS], iv[ROWS], val[ROWS][6];
-    unsigned col[ROWS][6];  // shared-memory address of the column's p (the zero slot when absent)
-    int slot[ROWS];
-};
-// ps: NT * ROWS + 4 floats in shared memory; slot NT * ROWS holds 0
 template <int ROWS, int NT>
-__device__ __forceinline__ void cg_rows_load(const DCoarsest& C, CgRows<ROWS>& M, const float* ps) {
-    const int tid = threadIdx.x, n = C.n;
+struct CgRows {
+    using S = CgShape<ROWS, NT>;
+    float val[S::R][6];
+    unsigned col[S::R][S::LEAN ? 3 : 6];  // shared-memory address of the column's p (the zero slot when absent)
+    float dg[S::LEAN ? 1 : S::R], iv[S::LEAN ? 1 : S::R];
+    int slot[S::LEAN ? 1 : S::R];
+};
+template <int ROWS, int NT>
+__device__ __forceinline__ int cg_row(int q) {  // the q-th row of this thread
+    return (int)threadIdx.x + (q / ROWS) * CG_THREADS + (q % ROWS) * NT;
+}
+// ps: SMEM_FLOATS floats in shared memory: p by row, the zero slot, then (lean) 1/diag, diag and x by row
+template <int ROWS, int NT>
+__device__ __forceinline__ void cg_rows_load(const DCoarsest& C, CgRows<ROWS, NT>& M, float* ps) {
+    using S = CgShape<ROWS, NT>;
+    const int n = C.n;
     const unsigned base = (unsigned)__cvta_generic_to_shared(ps);
+    float* siv = ps + S::N + 4;
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-        const int i = tid + k * NT;
+    for (int q = 0; q < S::R; ++q) {
+        const int i = cg_row<ROWS, NT>(q);
         const bool ok = i < n;
-        M.slot[k] = ok ? C.dof_slot[i] : -1;
-        M.dg[k] = ok ? C.diag[i] : 0.f;
-        M.iv[k] = ok ? C.invd[i] : 0.f;
+        if constexpr (S::LEAN) {
+            siv[i] = ok ? C.invd[i] : 0.f;
+            siv[S::N + i] = ok ? C.diag[i] : 0.f;
+        } else {
+            M.slot[q] = ok ? C.dof_slot[i] : -1;
+            M.dg[q] = ok ? C.diag[i] : 0.f;
+            M.iv[q] = ok ? C.invd[i] : 0.f;
+        }
 #pragma unroll
         for (int e = 0; e < 6; ++e) {
             const int c = ok ? C.col[i * 6 + e] : -1;
-            M.col[k][e] = base + 4u * (unsigned)(c >= 0 ? c : NT * ROWS);
-            M.val[k][e] = c >= 0 ? C.val[i * 6 + e] : 0.f;
+            const unsigned o = 4u * (unsigned)(c >= 0 ? c : S::N);
+            if constexpr (S::LEAN) M.col[q][e >> 1] = (e & 1) ? (M.col[q][e >> 1] | (o << 16)) : o;
+            else M.col[q][e] = base + o;
+            M.val[q][e] = c >= 0 ? C.val[i * 6 + e] : 0.f;
         }
     }
 }
@@ -1442,74 +1491,105 @@ __device__ __forceinline__ float lds_f32(unsigned addr) {
     return v;
 }
 // out[slot] = the 10-step CG solution for the rhs gathered from rhs[slot]
-// (every thread of the NT-thread block takes part); ps: NT * ROWS + 4 floats,
-// red: 16-byte aligned.  The products and sums use fused multiply-adds (the
-// coarsest solve's summation order is this kernel's own; the unfused
-// reference solve differs from it by rounding only).
+// (every thread of the CG_THREADS-thread block takes part); red: 16-byte
+// aligned.  The products and sums use fused multiply-adds (the coarsest
+// solve's summation order is this kernel's own; the unfused reference solve
+// differs from it by rounding only).
 template <int ROWS, int NT>
-__device__ __forceinline__ void cg_rows_solve(const CgRows<ROWS>& M, const float* rhs, float* out, float* ps,
-                                              float (*red)[64]) {
+__device__ __forceinline__ void cg_rows_solve(const DCoarsest& C, const CgRows<ROWS, NT>& M, const float* rhs,
+                                              float* out, float* ps, float (*red)[64]) {
+    using S = CgShape<ROWS, NT>;
+    constexpr int R = S::R, V = S::V;
     const int tid = threadIdx.x;
-    float x[ROWS], r[ROWS], p[ROWS], z[ROWS];
-    float bb = 0.f;
-    if (tid == 0) ps[NT * ROWS] = 0.f;  // the absent columns' slot (published by the first barrier)
+    const unsigned base = (unsigned)__cvta_generic_to_shared(ps);
+    float* siv = ps + S::N + 4;
+    float* sdg = siv + S::N;
+    float* sx = sdg + S::N;
+    float x[S::LEAN ? 1 : R], r[R], p[R];
+    auto inv = [&](int q) { return S::LEAN ? siv[cg_row<ROWS, NT>(q)] : M.iv[S::LEAN ? 0 : q]; };
+    float bb[V];
+    if (tid == 0) ps[S::N] = 0.f;  // the absent columns' slot (published by the first barrier)
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-        x[k] = 0.f;
-        r[k] = M.slot[k] >= 0 ? rhs[M.slot[k]] : 0.f;
-        bb = __fmaf_rn(r[k], r[k], bb);
+    for (int q = 0; q < R; ++q) {
+        const int i = cg_row<ROWS, NT>(q);
+        int slot;
+        if constexpr (S::LEAN) {
+            slot = i < C.n ? C.dof_slot[i] : -1;
+            sx[i] = 0.f;
+        } else {
+            slot = M.slot[q];
+            x[q] = 0.f;
+        }
+        r[q] = slot >= 0 ? rhs[slot] : 0.f;
+        bb[q / ROWS] = __fmaf_rn(r[q], r[q], q % ROWS ? bb[q / ROWS] : 0.f);
     }
     int rb = 0;
-    const float rhsNorm2 = cg_block_sum<NT>(bb, red[rb]);
+    const float rhsNorm2 = cg_block_sum<V>(bb, red[rb]);
     rb = rb == 2 ? 0 : rb + 1;
     const float threshold = fmaxf(__fmul_rn(__fmul_rn(FLT_EPSILON, FLT_EPSILON), rhsNorm2), FLT_MIN);
     // rhsNorm2 == 0 -> x = 0; residualNorm2 (== rhsNorm2 for x = 0) < threshold -> x = 0
     if (rhsNorm2 != 0.f && !(rhsNorm2 < threshold)) {
-        float an = 0.f;
+        float an[V];
 #pragma unroll
-        for (int k = 0; k < ROWS; ++k) {
-            p[k] = __fmul_rn(M.iv[k], r[k]);
-            an = __fmaf_rn(r[k], p[k], an);
+        for (int q = 0; q < R; ++q) {
+            p[q] = __fmul_rn(inv(q), r[q]);
+            an[q / ROWS] = __fmaf_rn(r[q], p[q], q % ROWS ? an[q / ROWS] : 0.f);
         }
-        float absNew = cg_block_sum<NT>(an, red[rb]);
+        float absNew = cg_block_sum<V>(an, red[rb]);
         rb = rb == 2 ? 0 : rb + 1;
         for (int it = 0; it < 10; ++it) {
 #pragma unroll
-            for (int k = 0; k < ROWS; ++k) ps[tid + k * NT] = p[k];
+            for (int q = 0; q < R; ++q) ps[cg_row<ROWS, NT>(q)] = p[q];
             __syncthreads();
-            float pt = 0.f, tq[ROWS];
+            float pt[V], tq[R];
 #pragma unroll
-            for (int k = 0; k < ROWS; ++k) {
-                float s = __fmul_rn(M.dg[k], p[k]);
+            for (int q = 0; q < R; ++q) {
+                float s = __fmul_rn(S::LEAN ? sdg[cg_row<ROWS, NT>(q)] : M.dg[S::LEAN ? 0 : q], p[q]);
 #pragma unroll
-                for (int e = 0; e < 6; ++e) s = __fmaf_rn(M.val[k][e], lds_f32(M.col[k][e]), s);
-                tq[k] = s;
-                pt = __fmaf_rn(p[k], s, pt);
+                for (int e = 0; e < 6; ++e) {
+                    unsigned a;
+                    if constexpr (S::LEAN) a = base + ((e & 1) ? (M.col[q][e >> 1] >> 16) : (M.col[q][e >> 1] & 0xffffu));
+                    else a = M.col[q][e];
+                    s = __fmaf_rn(M.val[q][e], lds_f32(a), s);
+                }
+                tq[q] = s;
+                pt[q / ROWS] = __fmaf_rn(p[q], s, q % ROWS ? pt[q / ROWS] : 0.f);
             }
-            const float alpha = __fdiv_rn(absNew, cg_block_sum<NT>(pt, red[rb]));
+            const float alpha = __fdiv_rn(absNew, cg_block_sum<V>(pt, red[rb]));
             rb = rb == 2 ? 0 : rb + 1;
-            float rr = 0.f, rz = 0.f;
+            float rr[V], rz[V];
 #pragma unroll
-            for (int k = 0; k < ROWS; ++k) {
-                x[k] = __fmaf_rn(alpha, p[k], x[k]);
-                r[k] = __fmaf_rn(-alpha, tq[k], r[k]);
-                z[k] = __fmul_rn(M.iv[k], r[k]);
-                rr = __fmaf_rn(r[k], r[k], rr);
-                rz = __fmaf_rn(r[k], z[k], rz);
+            for (int q = 0; q < R; ++q) {
+                if constexpr (S::LEAN) {
+                    float* xq = sx + cg_row<ROWS, NT>(q);
+                    *xq = __fmaf_rn(alpha, p[q], *xq);
+                } else {
+                    x[q] = __fmaf_rn(alpha, p[q], x[q]);
+                }
+                r[q] = __fmaf_rn(-alpha, tq[q], r[q]);
+                tq[q] = __fmul_rn(inv(q), r[q]);  // z
+                rr[q / ROWS] = __fmaf_rn(r[q], r[q], q % ROWS ? rr[q / ROWS] : 0.f);
+                rz[q / ROWS] = __fmaf_rn(r[q], tq[q], q % ROWS ? rz[q / ROWS] : 0.f);
             }
-            const float2 s2 = cg_block_sum2<NT>(rr, rz, red[rb]);
+            const float2 s2 = cg_block_sum2<V>(rr, rz, red[rb]);
             rb = rb == 2 ? 0 : rb + 1;
             if (s2.x < threshold) break;
             const float absOld = absNew;
             absNew = s2.y;
             const float beta = __fdiv_rn(absNew, absOld);
 #pragma unroll
-            for (int k = 0; k < ROWS; ++k) p[k] = __fmaf_rn(beta, p[k], z[k]);
+            for (int q = 0; q < R; ++q) p[q] = __fmaf_rn(beta, p[q], tq[q]);
         }
     }
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k)
-        if (M.slot[k] >= 0) out[M.slot[k]] = x[k];
+    for (int q = 0; q < R; ++q) {
+        const int i = cg_row<ROWS, NT>(q);
+        if constexpr (S::LEAN) {
+            if (i < C.n) out[C.dof_slot[i]] = sx[i];
+        } else {
+            if (M.slot[q] >= 0) out[M.slot[q]] = x[q];
+        }
+    }
 }
 
 // The whole coarsest solve.  WAIT: the body itself waits for the previous
@@ -1518,20 +1598,25 @@ __device__ __forceinline__ void cg_rows_solve(const CgRows<ROWS>& M, const float
 template <int ROWS, int NT, bool WAIT>
 __device__ __forceinline__ void coarsest_cg_body(const DCoarsest& C, const float* rhs, float* out, float* ps,
                                                  float (*red)[64]) {
-    CgRows<ROWS> M;
+    CgRows<ROWS, NT> M;
     cg_rows_load<ROWS, NT>(C, M, ps);
     if (WAIT) {
         griddep_wait();
         griddep_launch();
     }
-    cg_rows_solve<ROWS, NT>(M, rhs, out, ps, red);
+    cg_rows_solve<ROWS, NT>(C, M, rhs, out, ps, red);
 }
 
+// dynamic shared memory of a coarsest-CG launch
 template <int ROWS, int NT>
-__global__ void __launch_bounds__(NT, 1) k_coarsest_cg(DCoarsest C, const float* rhs, float* out) {
-    __shared__ float ps[NT * ROWS + 4];
+constexpr unsigned cg_smem_bytes() {
+    return (unsigned)CgShape<ROWS, NT>::SMEM_FLOATS * 4u;
+}
+template <int ROWS, int NT>
+__global__ void __launch_bounds__(CG_THREADS, 1) k_coarsest_cg(DCoarsest C, const float* rhs, float* out) {
+    extern __shared__ __align__(16) float cg_ps[];
     __shared__ __align__(16) float red[3][64];  // rotating reduction buffers (no reuse within 2 barriers)
-    coarsest_cg_body<ROWS, NT, true>(C, rhs, out, ps, red);
+    coarsest_cg_body<ROWS, NT, true>(C, rhs, out, cg_ps, red);
 }
 
 }  // namespace uaamg
