@@ -1,12 +1,14 @@
-"""The cluster kernel for the bottom of the pressure cycle against the launch
-sequence it replaces, at the sizes where its form changes (one or two leaves
-per thread, the three shapes of the coarsest CG), and the coarsest solves
-themselves against the oracle.  The kernel does the same operations in the same
-order: bit-identical."""
+"""The cluster kernels for the bottom of the cycles against the launch
+sequences they replace, at the sizes where their forms change: pressure
+(k_bottom: one or two leaves per thread, the three shapes of the coarsest CG)
+and viscosity (k_vbottom: level next to the coarsest as the top level or below
+it, the coarsest CG in one CTA or over eight, a level that does not fit), and
+the coarsest solves themselves against the oracle.  The kernels do the same
+operations in the same order: bit-identical."""
 import numpy as np
 import pytest
 
-from oracle.oracle import OraclePoisson
+from oracle.oracle import OraclePoisson, OracleViscosity
 from uaamg_b200 import scenes
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +68,39 @@ def test_pressure_coarsest_solve_of_each_shape(gpu):
         b[ref.dof_index(lc) < 0] = 0
         g, c = lap.coarsest_solve(b), ref.coarsest_solve(b)
         assert np.linalg.norm(g - c) <= 1e-4 * np.linalg.norm(c)
+
+
+# coarsest DOF: 884 under a top level of 5,668; 2,836 under 19,208; 880 under 5,836; 1,668 under 11,568; 2,520 under
+# 19,028; 3,852 under 29,948, which does not fit
+@pytest.mark.parametrize("n,fits", [(16, True), (24, True), (32, True), (40, True), (48, True), (56, False)])
+def test_viscosity_bottom_identical(gpu, monkeypatch, n, fits):
+    from uaamg_b200.viscosity import L_with_level, simd_viscosity3d
+    sc = scenes.plain_viscosity_scene(n=n, seed=2)
+    out = []
+    for on in ("0", "1"):
+        monkeypatch.setenv("UAAMG_VISC_BOTTOM", on)
+        lv = L_with_level.create_viscosity_matrix(sc.viscosity, sc.liquid_phi, sc.solid_phi, sc.dt, sc.rho, sc.dx)
+        rhs = lv.build_rhs(sc.u, sc.v, sc.w, sc.solid_velocity)
+        s = simd_viscosity3d(lv)
+        z = s.precondition(rhs)
+        x = lv.gather_velocity(sc.u, sc.v, sc.w)
+        st = s.pcg_solve(x, 1e-6, rhs)
+        d, d0 = gpu.from_numpy(rhs).cuda(), gpu.zeros(rhs.shape, device="cuda")
+        bottom = any("bottom" in k for k in s.profile_pcg(d0, d, 1e-6))
+        out.append((z, x, st, s.m_iteration, bottom))
+    (z0, x0, st0, it0, b0), (z1, x1, st1, it1, b1) = out
+    assert not b0 and b1 == fits
+    assert np.array_equal(z0, z1) and np.array_equal(x0, x1) and (st0, it0) == (st1, it1)
+
+
+@pytest.mark.parametrize("n", [24, 32, 56])
+def test_viscosity_coarsest_solve_bit_exact(gpu, n):
+    from uaamg_b200.viscosity import L_with_level
+    sc = scenes.plain_viscosity_scene(n=n, seed=2)
+    lv = L_with_level.create_viscosity_matrix(sc.viscosity, sc.liquid_phi, sc.solid_phi, sc.dt, sc.rho, sc.dx)
+    ref = OracleViscosity(sc.liquid_phi, sc.solid_phi, sc.viscosity, sc.dt, sc.rho, sc.dx)
+    lc = lv.num_levels() - 1
+    b = np.random.default_rng(61).uniform(-1, 1, ref.zeros(lc).shape).astype(np.float32)
+    b[ref.dof_index(lc) < 0] = 0
+    for rhs in (b, np.zeros_like(b)):
+        assert np.array_equal(lv.solve_exact(rhs), ref.coarsest_solve(rhs))

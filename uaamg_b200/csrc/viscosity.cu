@@ -14,6 +14,7 @@
 // shares its error handling, resource pools and launch helpers.
 #include <climits>
 
+#include "viscosity_bottom.cuh"
 #include "viscosity_build.cuh"
 
 namespace {
@@ -302,6 +303,10 @@ struct uaamg_viscosity {
     int* org0 = nullptr;
     float* zpage = nullptr;  // [512] zeros
     DCoarsestV C{};
+    // the level next to the coarsest by DOF and the shape of k_vbottom over it (bot_NC row CTAs, 0: not used)
+    VBotRows bot{};
+    int bot_NC = 0, bot_rows = 0;
+    size_t bot_smem = 0;
     float *x = nullptr, *b = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;
     double* partials = nullptr;
     PcgState* st = nullptr;
@@ -418,6 +423,79 @@ static void upload_defpage(uaamg_viscosity* h, VLevelDev& D) {
 static void upload_parents(uaamg_viscosity* h, const VHostLevel& H, VLevelDev& D) {
     D.L.parent = vupload(h, H.parent.data(), H.parent.size());
     D.L.octant = vupload(h, H.octant.data(), H.octant.size());
+}
+
+// k_vbottom's CG form by the coarsest system's size (rows per thread of a CTA of its own, 0: over eight CTAs)
+static int vbottom_cg_rows(int nc) { return nc <= 4 * VCG_THREADS ? 4 : 0; }
+static void (*vbottom_kernel(int rows))(VBotArgs) { return rows ? k_vbottom<4> : k_vbottom<0>; }
+// The rows of level nlev - 2 for k_vbottom, where it fits: 16-bit row numbers,
+// and a cluster whose CTAs hold their rows beside a copy of the whole vector
+// (up to about 20,000 DOF).  Row CTAs: enough that a pass gives a CTA at most
+// VB_PASS_ROWS rows (one per thread of half the block), more where the shared
+// memory asks for it.
+#define VB_PASS_ROWS 128
+static void build_vbottom(uaamg_viscosity* h) {
+    h->bot_NC = 0;
+    const char* off = getenv("UAAMG_VISC_BOTTOM");  // 0: the launch sequence
+    if (h->nlev < 2 || (off && off[0] == '0')) return;
+    const int lb = h->nlev - 2;
+    const VHostLevel& H = h->host[lb];
+    const int nc = h->C.n;
+    if (H.ndof <= 0 || H.ndof >= 65535 || nc <= 0) return;
+    VBotRows R{};
+    R.n = (int)H.ndof;
+    R.nc = nc;
+    std::vector<int32_t> base((size_t)H.nl * 6);
+    int acc = 0, most = 0;
+    for (int g = 0; g < 6; ++g) {
+        R.gs[g] = acc;
+        for (int i = 0; i < H.nl; ++i) {
+            base[(size_t)i * 6 + g] = acc;
+            const uint64_t* m = &H.dof[((size_t)(g >> 1) * H.nl + i) * 8];
+            for (int w = 0; w < 8; ++w) acc += __builtin_popcountll(m[w] & vcolour_mask(w, g & 1));
+        }
+        most = std::max(most, acc - R.gs[g]);
+    }
+    R.gs[6] = acc;
+    const int rows = vbottom_cg_rows(nc);
+    const int hi = VB_MAX_CLUSTER - (rows ? 1 : 0), lo = rows ? 1 : VB_CG8;
+    int optin = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->ctx->device));
+    const int max_dynamic = optin - 6 * 1024;  // above the kernel's static shared memory
+    int NC = std::min(hi, std::max(lo, (most + VB_PASS_ROWS - 1) / VB_PASS_ROWS));
+    size_t smem = 0;
+    for (;; ++NC) {
+        if (NC > hi) return;
+        int cap = 0;
+        for (int g = 0; g < 6; ++g) cap += (R.gs[g + 1] - R.gs[g] + NC - 1) / NC;
+        smem = (rows ? vbot_layout<4>(R.n, nc, cap) : vbot_layout<0>(R.n, nc, cap)).total;
+        if (smem <= (size_t)max_dynamic) break;
+    }
+    if (!cluster_fits(vbottom_kernel(rows), NC + (rows ? 1 : 0), VB_THREADS, smem, max_dynamic)) return;
+    const size_t n = (size_t)R.n;
+    int* dbase = vupload(h, base.data(), base.size());
+    float* coef = (float*)valloc(h, n * VB_COEF * 4);
+    unsigned* idx = (unsigned*)valloc(h, n * (VB_COEF / 2) * 4);
+    float* iv = (float*)valloc(h, n * 4);
+    float* dg = (float*)valloc(h, n * 4);
+    int* slot = (int*)valloc(h, n * 4);
+    uint16_t* cdst = (uint16_t*)valloc(h, n * 2);
+    int* rcount = (int*)valloc(h, VB_CG8 * 4);
+    CK(cudaMemsetAsync(rcount, 0, VB_CG8 * 4, h->stream));
+    const VLevelDev &D = h->lv[lb], &P = h->lv[lb + 1];
+    launch2(k_vbot_rows, dim3((unsigned)D.L.nl, 3, 4), 128, h->stream, D.L, P.L, (const int*)dbase,
+            (const int*)P.dof_base, R.n, coef, idx, iv, dg, slot, cdst, rcount);
+    R.coef = coef;
+    R.idx = idx;
+    R.iv = iv;
+    R.dg = dg;
+    R.slot = slot;
+    R.cdst = cdst;
+    R.rcount = rcount;
+    h->bot = R;
+    h->bot_NC = NC;
+    h->bot_rows = rows;
+    h->bot_smem = smem;
 }
 
 static void build_viscosity(uaamg_viscosity* h, const uaamg_leaf_grid* mu_g, const uaamg_leaf_grid* liq,
@@ -594,6 +672,7 @@ static void build_viscosity(uaamg_viscosity* h, const uaamg_leaf_grid* mu_g, con
         h->C.invd = invd;
         h->C.slot = slot;
     }
+    build_vbottom(h);
     // PCG vectors and scalars
     {
         const size_t vb = (size_t)3 * h->host[0].nl * UAAMG_LEAF * 4;
@@ -731,11 +810,26 @@ struct VEnq {
     void coarsest(const float* rhs, float* out) {
         if (h->C.n == 0) return;
         if (prof) pb("coarsest cg");
-        const int n = h->C.n;
-        if (n <= 2 * VCG_THREADS) launch2(k_vcoarsest_cg<2>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
-        else if (n <= 4 * VCG_THREADS) launch2(k_vcoarsest_cg<4>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
-        else if (n <= 8 * VCG_THREADS) launch2(k_vcoarsest_cg<8>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
-        else launch2(k_vcoarsest_cg<16>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
+        if (h->C.n <= 2 * VCG_THREADS) launch2(k_vcoarsest_cg<2>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
+        else if (vbottom_cg_rows(h->C.n)) launch2(k_vcoarsest_cg<4>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
+        else launch_cluster(k_vcoarsest_cg8, VB_CG8, VB_THREADS, vcg8_smem_bytes(h->C.n), s, h->C, rhs, out, &h->st->error);
+        pe();
+        count++;
+    }
+    // the visits of level nlev - 2 with their coarsest solves in one cluster launch (both of a W-cycle's visits; one
+    // when it is the top level), from a zero guess
+    void bottom(float* lhs, const float* rhs) {
+        VBotArgs A;
+        memset(&A, 0, sizeof(A));  // padding included: the recorder compares argument bytes
+        A.R = h->bot;
+        A.C = h->C;
+        A.NC = h->bot_NC;
+        A.visits = h->nlev == 2 ? 1 : 2;
+        A.rhs = rhs;
+        A.lhs = lhs;
+        A.error = &h->st->error;
+        if (prof) pb("L" + std::to_string(h->nlev - 2) + " bottom (visits + coarsest)");
+        launch_cluster(vbottom_kernel(h->bot_rows), h->bot_NC + (h->bot_rows ? 1 : 0), VB_THREADS, h->bot_smem, s, A);
         pe();
         count++;
     }
@@ -758,14 +852,19 @@ static void enqueue_mucycle(VEnq& E, int l, float* lhs, const float* rhs, bool f
         E.coarsest(rhs, lhs);
         return;
     }
+    if (l == h->nlev - 2 && h->bot_NC) {
+        E.bottom(lhs, rhs);
+        return;
+    }
     if (for_precon && !lhs_zeroed) E.zero(l, lhs);
     E.rbgs2(l, true, lhs, rhs);
     VLevelDev& D = h->lv[l];
     VLevelDev& P = h->lv[l + 1];
-    const bool coarse_visit = l + 1 != h->nlev - 1;  // the coarsest solve writes its own result
+    const bool bottom = l + 1 == h->nlev - 2 && h->bot_NC;  // both visits at once, from zero
+    const bool coarse_visit = l + 1 != h->nlev - 1 && !bottom;  // the coarsest solve writes its own result
     E.residual_restrict(l, lhs, rhs, P.rhs, coarse_visit ? P.lhs : nullptr);
     enqueue_mucycle(E, l + 1, P.lhs, P.rhs, true, coarse_visit);
-    if (l + 1 != h->nlev - 1) enqueue_mucycle(E, l + 1, P.lhs, P.rhs, false);
+    if (coarse_visit) enqueue_mucycle(E, l + 1, P.lhs, P.rhs, false);
     E.prolong(l, P.lhs, lhs);
     E.rbgs2(l, false, lhs, rhs);
 }

@@ -1302,10 +1302,10 @@ struct DCoarsestV {
 // Restatement of Eigen::ConjugateGradient (Upper|Lower, diagonal
 // preconditioner, tolerance FLT_EPSILON, maxIterations 10, zero guess) on the
 // coarsest level, one CTA of VCG_THREADS threads: row i = tid + k *
-// VCG_THREADS, ROWS rows per thread.  With ROWS <= 4 a thread keeps its rows'
-// ELL entries in registers for the whole solve; more rows read them through
-// L1.  Few warps keep the three barriers and two reductions of an iteration
-// short.
+// VCG_THREADS, ROWS rows per thread, whose ELL entries stay in registers for
+// the whole solve (up to 4 rows; larger systems are solved by eight CTAs in the
+// same order, vcg8_solve).  Few warps keep the three barriers and two
+// reductions of an iteration short.
 #define VCG_THREADS 256
 #define VCG_WARPS (VCG_THREADS / 32)
 // Block sums in one barrier: a shuffle-down tree inside each warp, then every
@@ -1331,46 +1331,43 @@ __device__ __forceinline__ float2 vcg_block_sum2(float a, float b, float* buf) {
     return make_float2(cg_tree_sum<VCG_WARPS>(buf), cg_tree_sum<VCG_WARPS>(buf + 32));
 }
 
-// Rows of ROWS <= 4 stay in registers with the shared-memory address of each
-// entry's p (padding entries: value 0 at a slot that holds 0); larger systems
-// read their rows from global memory each iteration.  A row's product is
+// A thread's rows with the shared-memory address of each entry's p (padding
+// entries: value 0 at a slot that holds 0).  A row's product is
 // s = fma(v_e, p[c_e], s) over its VCG_W entries, padding included.
 template <int ROWS>
-__global__ void __launch_bounds__(VCG_THREADS, 1) k_vcoarsest_cg(DCoarsestV C, const float* rhs, float* out) {
-    constexpr bool REG = ROWS <= 4;
-    constexpr int ZERO = VCG_THREADS * ROWS;  // the zero slot
-    __shared__ float ps[VCG_THREADS * ROWS + 4];
-    __shared__ __align__(16) float red[3][64];
+struct VCgRows {
+    float iv[ROWS], val[ROWS][VCG_W];
+    unsigned col[ROWS][VCG_W];
+};
+// ps: VCG_THREADS * ROWS + 4 floats, the last four the zero slot
+template <int ROWS>
+__device__ __forceinline__ void vcg_load(const DCoarsestV& C, VCgRows<ROWS>& M, float* ps) {
     const int tid = threadIdx.x, n = C.n;
+    constexpr int ZERO = VCG_THREADS * ROWS;
     const unsigned psb = (unsigned)__cvta_generic_to_shared(ps);
-    float x[ROWS], r[ROWS], p[ROWS], z[ROWS], iv[ROWS];
-    unsigned rc[REG ? ROWS : 1][VCG_W];
-    float rv[REG ? ROWS : 1][VCG_W];
-    long long sl[ROWS];
-    // static data (rows, 1/diag, slots) before the wait for rhs
 #pragma unroll
     for (int k = 0; k < ROWS; ++k) {
         const int i = tid + k * VCG_THREADS;
-        sl[k] = i < n ? C.slot[i] : -1;
-        iv[k] = i < n ? C.invd[i] : 0.f;
-        if (REG) {
+        M.iv[k] = i < n ? C.invd[i] : 0.f;
 #pragma unroll
-            for (int e = 0; e < VCG_W; ++e) {
-                const int cc = i < n ? __ldg(C.col + (long long)i * VCG_W + e) : -1;
-                rc[REG ? k : 0][e] = psb + 4u * (unsigned)(cc >= 0 ? cc : ZERO);
-                rv[REG ? k : 0][e] = cc >= 0 ? __ldg(C.val + (long long)i * VCG_W + e) : 0.f;
-            }
+        for (int e = 0; e < VCG_W; ++e) {
+            const int cc = i < n ? __ldg(C.col + (long long)i * VCG_W + e) : -1;
+            M.col[k][e] = psb + 4u * (unsigned)(cc >= 0 ? cc : ZERO);
+            M.val[k][e] = cc >= 0 ? __ldg(C.val + (long long)i * VCG_W + e) : 0.f;
         }
     }
     if (tid == 0) ps[ZERO] = 0.f;  // published by the first reduction's barrier
-    griddep_wait();
-    griddep_launch();
+}
+// x of the thread's rows for the rhs r (0 in rows that do not exist; overwritten)
+template <int ROWS>
+__device__ __forceinline__ void vcg_solve(const VCgRows<ROWS>& M, float (&r)[ROWS], float (&x)[ROWS], float* ps,
+                                          float (*red)[64]) {
+    const int tid = threadIdx.x;
+    float p[ROWS], z[ROWS];
     float bb = 0.f;
 #pragma unroll
     for (int k = 0; k < ROWS; ++k) {
         x[k] = 0.f;
-        r[k] = sl[k] >= 0 ? rhs[sl[k]] : 0.f;
-        p[k] = 0.f;
         bb = __fmaf_rn(r[k], r[k], bb);
     }
     int rb = 0;
@@ -1381,7 +1378,7 @@ __global__ void __launch_bounds__(VCG_THREADS, 1) k_vcoarsest_cg(DCoarsestV C, c
         float an = 0.f;
 #pragma unroll
         for (int k = 0; k < ROWS; ++k) {
-            p[k] = __fmul_rn(iv[k], r[k]);
+            p[k] = __fmul_rn(M.iv[k], r[k]);
             an = __fmaf_rn(r[k], p[k], an);
         }
         float absNew = vcg_block_sum(an, red[rb]);
@@ -1393,20 +1390,9 @@ __global__ void __launch_bounds__(VCG_THREADS, 1) k_vcoarsest_cg(DCoarsestV C, c
             float pt = 0.f, tq[ROWS];
 #pragma unroll
             for (int k = 0; k < ROWS; ++k) {
-                const int i = tid + k * VCG_THREADS;
                 float s = 0.f;
-                if (REG) {
 #pragma unroll
-                    for (int e = 0; e < VCG_W; ++e) s = __fmaf_rn(rv[REG ? k : 0][e], lds_f32(rc[REG ? k : 0][e]), s);
-                } else if (i < n) {
-                    const int* cr = C.col + (long long)i * VCG_W;
-                    const float* vr = C.val + (long long)i * VCG_W;
-#pragma unroll
-                    for (int e = 0; e < VCG_W; ++e) {
-                        const int cc = __ldg(cr + e);
-                        s = __fmaf_rn(cc >= 0 ? __ldg(vr + e) : 0.f, ps[cc >= 0 ? cc : ZERO], s);
-                    }
-                }
+                for (int e = 0; e < VCG_W; ++e) s = __fmaf_rn(M.val[k][e], lds_f32(M.col[k][e]), s);
                 tq[k] = s;
                 pt = __fmaf_rn(p[k], s, pt);
             }
@@ -1417,7 +1403,7 @@ __global__ void __launch_bounds__(VCG_THREADS, 1) k_vcoarsest_cg(DCoarsestV C, c
             for (int k = 0; k < ROWS; ++k) {
                 x[k] = __fmaf_rn(alpha, p[k], x[k]);
                 r[k] = __fmaf_rn(-alpha, tq[k], r[k]);
-                z[k] = __fmul_rn(iv[k], r[k]);
+                z[k] = __fmul_rn(M.iv[k], r[k]);
                 rr = __fmaf_rn(r[k], r[k], rr);
                 rz = __fmaf_rn(r[k], z[k], rz);
             }
@@ -1431,6 +1417,26 @@ __global__ void __launch_bounds__(VCG_THREADS, 1) k_vcoarsest_cg(DCoarsestV C, c
             for (int k = 0; k < ROWS; ++k) p[k] = __fmaf_rn(beta, p[k], z[k]);
         }
     }
+}
+template <int ROWS>
+__global__ void __launch_bounds__(VCG_THREADS, 1) k_vcoarsest_cg(DCoarsestV C, const float* rhs, float* out) {
+    __shared__ float ps[VCG_THREADS * ROWS + 4];
+    __shared__ __align__(16) float red[3][64];
+    VCgRows<ROWS> M;
+    long long sl[ROWS];
+    // static data before the wait for rhs
+    vcg_load<ROWS>(C, M, ps);
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+        const int i = (int)threadIdx.x + k * VCG_THREADS;
+        sl[k] = i < C.n ? C.slot[i] : -1;
+    }
+    griddep_wait();
+    griddep_launch();
+    float r[ROWS], x[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) r[k] = sl[k] >= 0 ? rhs[sl[k]] : 0.f;
+    vcg_solve<ROWS>(M, r, x, ps, red);
 #pragma unroll
     for (int k = 0; k < ROWS; ++k)
         if (sl[k] >= 0) out[sl[k]] = x[k];
