@@ -111,7 +111,7 @@ int uaamg_poisson_create_with_rhs(const uaamg_leaf_grid* liquid_phi, const uaamg
 typedef struct {
     int32_t staged_min_leaves;  /* levels of at least this many leaves sweep with the bulk-copy staged kernels (64) */
     int32_t split_min_leaves;   /* ... store a computed source (first sweep, prolongation) before sweeping (1024) */
-    int32_t pipe_min_leaves;    /* ... sweep and restrict with the persistent pipelined kernels (8192) */
+    int32_t pipe_min_leaves;    /* ... sweep with the marching kernels (1024) */
     int32_t elem_ctas_per_sm;   /* CTAs per SM of the grid-stride passes, 1..32 (16) */
     int32_t bottom_cycle;       /* 1: both visits of the level above the coarsest, with the coarsest solves, as one
                                  * thread-block-cluster launch where the level fits (1) */

@@ -22,7 +22,7 @@ candidate settings on representative solves and keeps the fastest:
   the library starts from its built-in defaults.
 
 ``pipe_min_leaves`` moves only the passes without a dot product: the passes
-that carry the PCG's level-0 dot products switch to the pipelined kernels at a
+that carry the PCG's level-0 dot products switch to the marching kernels at a
 fixed size (their per-CTA partials set the summation order), so no setting
 changes a result.
 

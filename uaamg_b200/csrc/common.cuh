@@ -20,6 +20,9 @@
 #define TRIM_Y 4u
 #define TRIM_Z 8u
 #define TRIM_SPAI0 16u
+// every voxel of the leaf is a DOF and every coefficient its stencils read, its
+// neighbours' included, is the default (set for large levels by k_plain_leaves)
+#define LEAF_PLAIN 32u
 
 // PCG status word
 #define PCG_RUNNING 0

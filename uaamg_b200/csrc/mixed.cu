@@ -197,9 +197,9 @@ struct MEnq {
         pe();
     }
     template <typename... KArgs, typename... Args>
-    void run_pipe(const char* what, int l, void (*kern)(KArgs...), int nl, size_t smem, Args... args) {
+    void run_march(const char* what, int l, int NP, void (*kern)(KArgs...), int nl, Args... args) {
         pb(what, l);
-        launch_pipe(kern, nl, smem, s, args...);
+        launch_march(kern, nl, NP, s, args...);
         pe();
     }
 };
@@ -211,6 +211,9 @@ struct MEnq {
 // STAGED_MIN_LEAVES leaves sweep with the staged kernels, and from
 // SPLIT_MIN_LEAVES on the first sweep's source and the prolongation-add are
 // stored first (k_mmaterialize) so that every sweep is a staged plain one.
+// 16-bit levels march from this size on (smaller ones: the one-leaf staged
+// kernels, as at PIPE_MIN_LEAVES).
+#define MARCH_MIN_LEAVES_16 1024
 template <typename T>
 static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     uaamg_poisson* h = E.h;
@@ -248,12 +251,13 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     const bool staged = g_use_staged && L.nl >= STAGED_MIN_LEAVES;
     const bool split = g_use_staged && L.nl >= SPLIT_MIN_LEAVES;
     int* err = &h->st->error;
-    const size_t psm = pipe_smem_bytes<MLevel<T>>();
-    const bool pipe = staged && L.nl >= PIPE_DOT_MIN_LEAVES;
+    const bool march = staged && L.nl >= MARCH_MIN_LEAVES_16, march_dot = staged && L.nl >= PIPE_DOT_MIN_LEAVES;
+    const int NP = march_planes(L.nl);
     auto sweep = [&](const T* x, T* out, float w) {  // plain source
-        if (pipe)
-            E.run_pipe("jacobi staged", l, k_pipe<M_JACOBI, MLevel<T>, T, false>, L.nl, psm, L, x, (const T*)rhs, out,
-                       w, 0.f, 0.f, nodot, ns, 0.f, err);
+        if (march)
+            E.run_march("jacobi staged", l, NP, NP == 8 ? k_march<M_JACOBI, MLevel<T>, T, false, 8>
+                                                        : k_march<M_JACOBI, MLevel<T>, T, false, 2>,
+                        L.nl, L, x, (const T*)rhs, out, w, 0.f, 0.f, nodot, ns, 0.f);
         else if (staged)
             E.run("jacobi staged", l, k_msweep_staged<T, T>, g, 128, L, x, (const T*)rhs, out, w, nodot, ns, err);
         else
@@ -277,9 +281,10 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     }
     const float cics = 1.0f / level_scale(h->lv[l + 1].L);
     T* crhs = (T*)M->lv[l + 1].rhs;
-    if (pipe)  // the pipelined kernel computes in stored units: its scale is cs / cs'
-        E.run_pipe("restrict staged", l, k_pipe<M_RESIDUAL, MLevel<T>, T, true>, L.nl, psm, L, (const T*)tmp,
-                   (const T*)rhs, crhs, 0.f, 0.f, 0.f, nodot, ns, L.cs * cics, err);
+    if (march)  // the marching kernel computes in stored units: its scale is cs / cs'
+        E.run_march("restrict staged", l, NP, NP == 8 ? k_march<M_RESIDUAL, MLevel<T>, T, true, 8>
+                                                      : k_march<M_RESIDUAL, MLevel<T>, T, true, 2>,
+                    L.nl, L, (const T*)tmp, (const T*)rhs, crhs, 0.f, 0.f, 0.f, nodot, ns, L.cs * cics);
     else if (staged)
         E.run("restrict staged", l, k_mrestrict_staged<T>, g, 128, L, (const T*)tmp, (const T*)rhs, crhs, cics, err);
     else
@@ -297,9 +302,10 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     }
     sweep(lhs, tmp, wpre(1));
     if (l == 0) {
-        if (pipe)
-            E.run_pipe("jacobi staged to fp32 +dot", l, k_pipe<M_JACOBI, MLevel<T>, float, false>, L.nl, psm, L,
-                       (const T*)tmp, (const T*)rhs, z, wpre(0), 0.f, 0.f, dot, (const float*)M->sigma, 0.f, err);
+        if (march_dot)
+            E.run_march("jacobi staged to fp32 +dot", l, NP, NP == 8 ? k_march<M_JACOBI, MLevel<T>, float, false, 8>
+                                                                     : k_march<M_JACOBI, MLevel<T>, float, false, 2>,
+                        L.nl, L, (const T*)tmp, (const T*)rhs, z, wpre(0), 0.f, 0.f, dot, (const float*)M->sigma, 0.f);
         else if (staged)
             E.run("jacobi staged to fp32 +dot", l, k_msweep_staged<T, float>, g, 128, L, (const T*)tmp,
                   (const T*)rhs, z, wpre(0), dot, (const float*)M->sigma, err);

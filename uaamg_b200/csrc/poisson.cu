@@ -30,7 +30,7 @@
 #include "common.cuh"
 #include "poisson_build.cuh"
 #include "poisson_kernels.cuh"
-#include "staged_pipe.cuh"
+#include "poisson_march.cuh"
 #include "poisson_bottom.cuh"
 #include "resources.cuh"
 
@@ -582,6 +582,8 @@ static LevelOut level_out(LevelDev& d) {
 
 }  // namespace
 
+// Levels of at least this many leaves have their plain leaves marked for the marching sweeps.
+#define PLAIN_MIN_LEAVES 64
 // ---------------------------------------------------------------------------
 // hierarchy construction
 #include <chrono>
@@ -957,6 +959,13 @@ static void build_hierarchy(uaamg_poisson* h, const uaamg_leaf_grid* phi, const 
             CHECK_LAUNCH();
             h->launches++;
         }
+        for (int l = 0; l < nlev; ++l) {
+            LevelDev& D = h->lv[l];
+            if (D.L.nl < PLAIN_MIN_LEAVES) continue;
+            k_plain_leaves<<<(unsigned)((D.L.nl + 127) / 128), 128, 0, s>>>(D.L, D.flags);
+            CHECK_LAUNCH();
+            h->launches++;
+        }
         // the rhs and the velocities' buffers: done before the inputs are freed and the handle is used
         if (ri) CK(cudaStreamWaitEvent(s, ev_vel.e, 0));
         for (void* pmem : tofree) CK(ctx_dev_free(h->ctx, pmem, s));
@@ -1000,7 +1009,7 @@ static bool g_use_sweep2 = true;  // fused Jacobi sweep pairs (Enq::pair)
 // table an autotuner wrote.  Every choice gives the same results; only the
 // speed differs.  g_tune_gen is part of every graph's key, so a change rebuilds
 // cached graphs.
-static uaamg_tuning g_tune = {64, 1024, 8192, 16, 1};
+static uaamg_tuning g_tune = {64, 1024, 1024, 16, 1};
 static int g_tune_gen = 0;
 static int g_sms = 148;  // SMs of the device (set when a handle is created)
 #define STAGED_MIN_LEAVES (g_tune.staged_min_leaves)
@@ -1012,14 +1021,23 @@ static int g_sms = 148;  // SMs of the device (set when a handle is created)
 // stored values are the ones the fused kernel computes, so the results are
 // identical.
 #define SPLIT_MIN_LEAVES (g_tune.split_min_leaves)
-// Levels of at least PIPE_MIN_LEAVES leaves sweep with the persistent
-// pipelined kernels (several leaves per CTA); smaller staged levels with the
-// one-leaf staged kernels, which start faster.
+// Sweeps of a stored source march from PIPE_MIN_LEAVES leaves on
+// (poisson_march.cuh); smaller staged levels use the one-leaf staged kernels,
+// whose four times as many warps hide more of a small level's latency.
+// Measured, Jacobi, marching / staged: 1,916 leaves 9.2 / 10.2 us, 284 leaves
+// 7.9 / 7.9 us.  Residual + restriction marches on every staged level.
 #define PIPE_MIN_LEAVES (g_tune.pipe_min_leaves)
+// Planes a half-warp marches: two (four times the warps, each plane along x
+// read twice) or a whole leaf.  A pass that ends in a reduction or stores an
+// eighth gains from fewer warps first, a 16-bit one as well; an FP32 sweep only
+// where DRAM bounds it.  Two / eight planes, us, at 20,500, 30,492, 51,000 and
+// 124,644 leaves: A p 49 / 42, 73 / 60, 117 / 88, 251 / 168; restriction
+// 34 / 36, 51 / 50, 79 / 72, 167 / 142; sweep 37 / 44, 56 / 60, 88 / 89,
+// 187 / 177; 16-bit sweep at 30,492: 54 / 49.
+static int march_planes(int nl, bool fp32_sweep = false) { return nl >= (fp32_sweep ? 65536 : 24576) ? 8 : 2; }
 // A pass that carries a level-0 dot product (the last post-smoothing sweep
-// with z.r, A p with p.q) uses the pipelined kernel from this fixed size on:
-// its per-CTA partials set the dot's summation order, which must not depend
-// on the tuning.  The mixed-precision form uses it for all its passes.
+// with z.r, A p with p.q) marches from this fixed size on: its per-CTA
+// partials set the dot's summation order, which must not depend on the tuning.
 #define PIPE_DOT_MIN_LEAVES 8192
 // Grid of the grid-stride elementwise kernels (k_materialize, the PCG
 // vector updates): 16 CTAs of 128 threads per SM of a 148-SM B200, at most
@@ -1144,11 +1162,10 @@ static bool cluster_fits(void (*kern)(KArgs...), int C, unsigned block, size_t s
     return n >= 1;
 }
 
-// Launch of a pipelined staged kernel (staged_pipe.cuh) over nl leaves:
-// PIPE_CTAS CTAs, at most one per leaf.
+// Launch of a marching sweep (poisson_march.cuh) over nl leaves, NP planes per half-warp.
 template <typename... KArgs, typename... Args>
-static void launch_pipe(void (*kern)(KArgs...), int nl, size_t smem, cudaStream_t s, Args... args) {
-    launch_smem(kern, (unsigned)std::min(nl, PIPE_CTAS), 128, smem, s, args...);
+static void launch_march(void (*kern)(KArgs...), int nl, int NP, cudaStream_t s, Args... args) {
+    launch(kern, march_grid(nl, NP), MARCH_THREADS, s, args...);
 }
 
 // Optional per-kernel timing (diagnostics): a CUDA event pair around every launch.
@@ -1227,11 +1244,15 @@ struct Enq {
         if constexpr (std::is_same<Src, SrcPlain>::value) {
             if (g_use_staged && D.L.nl >= STAGED_MIN_LEAVES && !(MODE == M_SPAI0 && mark_spai0)) {
                 if (prof) pb("L" + std::to_string(l) + " " + mode_name(MODE) + " staged" + (dot.r ? "+dot" : ""));
-                if (D.L.nl >= (dot.r ? PIPE_DOT_MIN_LEAVES : PIPE_MIN_LEAVES))
-                    launch_pipe(k_pipe<MODE, DLevel, float, false>, D.L.nl, pipe_smem_bytes<DLevel>(), s, D.L,
-                                (const float*)src.x, b, out, w, ws, 1.0f - ws, dot, (const float*)nullptr, 0.f,
-                                &h->st->error);
-                else
+                if (D.L.nl >= (dot.r ? PIPE_DOT_MIN_LEAVES : PIPE_MIN_LEAVES)) {
+                    auto go = [&](auto kern, int NP) {
+                        launch_march(kern, D.L.nl, NP, s, D.L, (const float*)src.x, b, out, w, ws, 1.0f - ws, dot,
+                                     (const float*)nullptr, 0.f);
+                    };
+                    const int NP = march_planes(D.L.nl, !dot.r);
+                    if (NP == 8) go(k_march<MODE, DLevel, float, false, 8>, 8);
+                    else go(k_march<MODE, DLevel, float, false, 2>, 2);
+                } else
                     launch(k_sweep_staged<MODE>, (unsigned)D.L.nl, 128, s, D.L, (const float*)src.x, b, out, w, ws,
                            1.0f - ws, dot, &h->st->error);
                 pe();
@@ -1274,12 +1295,13 @@ struct Enq {
         LevelDev& D = h->lv[l];
         if (g_use_staged && D.L.nl >= STAGED_MIN_LEAVES) {
             if (prof) pb("L" + std::to_string(l) + " residual+restrict staged");
-            if (D.L.nl >= PIPE_MIN_LEAVES)
-                launch_pipe(k_pipe<M_RESIDUAL, DLevel, float, true>, D.L.nl, pipe_smem_bytes<DLevel>(), s, D.L, x,
-                            b, h->lv[l + 1].rhs, 0.f, 0.f, 0.f, DotOut{nullptr, nullptr, nullptr},
-                            (const float*)nullptr, 0.f, &h->st->error);
-            else
-                launch(k_restrict_staged, (unsigned)D.L.nl, 128, s, D.L, x, b, h->lv[l + 1].rhs, &h->st->error);
+            auto go = [&](auto kern, int NP) {
+                launch_march(kern, D.L.nl, NP, s, D.L, x, b, h->lv[l + 1].rhs, 0.f, 0.f, 0.f,
+                             DotOut{nullptr, nullptr, nullptr}, (const float*)nullptr, 0.f);
+            };
+            const int NP = march_planes(D.L.nl);
+            if (NP == 8) go(k_march<M_RESIDUAL, DLevel, float, true, 8>, 8);
+            else go(k_march<M_RESIDUAL, DLevel, float, true, 2>, 2);
             pe();
             count++;
             return;
@@ -1579,16 +1601,18 @@ static void enqueue_setup(Enq& E, cudaGraphConditionalHandle cond, int use_cond)
     E.pe();
     E.count += 3;
 }
-// PCG lines 6-7: q = A p with sigma = p.q and alpha (pipelined staged kernel
+// PCG lines 6-7: q = A p with sigma = p.q and alpha (marching kernel
 // on large levels)
 static void enqueue_Ap(Enq& E) {
     uaamg_poisson* h = E.h;
     LevelDev& D0 = h->lv[0];
-    if (g_use_staged && D0.L.nl >= PIPE_DOT_MIN_LEAVES)
-        launch_pipe(k_pipe<M_LAPLACIAN, DLevel, float, false, 1>, D0.L.nl, pipe_smem_bytes<DLevel>(), E.s, D0.L,
-                    (const float*)h->p, (const float*)nullptr, h->q, 0.f, 0.f, 0.f,
-                    DotOut{h->p, h->partials, h->st}, (const float*)nullptr, 0.f, &h->st->error);
-    else
+    if (g_use_staged && D0.L.nl >= PIPE_DOT_MIN_LEAVES) {
+        const int NP = march_planes(D0.L.nl);
+        launch_march(NP == 8 ? k_march<M_LAPLACIAN, DLevel, float, false, 8, 1>
+                             : k_march<M_LAPLACIAN, DLevel, float, false, 2, 1>,
+                     D0.L.nl, NP, E.s, D0.L, (const float*)h->p, (const float*)nullptr, h->q, 0.f, 0.f, 0.f,
+                     DotOut{h->p, h->partials, h->st}, (const float*)nullptr, 0.f);
+    } else
         launch(k_pcg_Ap, (unsigned)D0.L.nl, 128, E.s, D0.L, (const float*)h->p, h->q, h->partials, h->st);
 }
 static void enqueue_body(Enq& E, cudaGraphConditionalHandle cond, int use_cond) {

@@ -1006,42 +1006,6 @@ __global__ void __launch_bounds__(128, STAGED_MINB) k_sweep_staged(DLevel L, con
     }
 }
 
-// residual + restriction with the fine leaf staged
-__global__ void __launch_bounds__(128, STAGED_MINB) k_restrict_staged(DLevel L, const float* x, const float* b, float* coarse,
-                                                         int* err) {
-    STAGED_SMEM_DECL
-    const int leaf = blockIdx.x, t = threadIdx.x;
-    unsigned fl;
-    float4 hxp, hxm, hyp, hym, hcxp, hcyp;
-    float hz, hcz;
-    const bool ok =
-        staged_prologue<M_RESIDUAL>(L, leaf, t, x, b, S, &sm_bar, fl, hxp, hxm, hyp, hym, hcxp, hcyp, hz, hcz, err);
-    if (!ok) return;
-    float4 xc;
-    unsigned m;
-    float4 r = staged_value<M_RESIDUAL>(L, leaf, t, fl, S, hxp, hxm, hyp, hym, hcxp, hcyp, hz, hcz, 0.f, 0.f, 0.f, xc, m);
-    __syncthreads();  // every thread has read sm_x before it is reused for the residuals
-    reinterpret_cast<float4*>(sm_x)[t] = r;
-    __syncthreads();
-    if (t < 64) {
-        const int i = t >> 4, j = (t >> 2) & 3, k = t & 3;
-        const uint64_t* mk = L.mask + (long long)leaf * 8;
-        float s = 0.f;
-#pragma unroll
-        for (int ii = 0; ii < 2; ++ii)
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-                    int fo = ((2 * i + ii) << 6) | ((2 * j + jj) << 3) | (2 * k + kk);
-                    if ((mk[fo >> 6] >> (fo & 63)) & 1ull) s = __fadd_rn(s, sm_x[fo]);
-                }
-        const int o = L.octant[leaf];
-        const int coff = ((((o >> 2) & 1) * 4 + i) << 6) | ((((o >> 1) & 1) * 4 + j) << 3) | ((o & 1) * 4 + k);
-        coarse[(long long)L.parent[leaf] * UAAMG_LEAF + coff] = __fmul_rn(s, 0.125f);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // PCG vector kernels (PoissonSolver::solveMultigridPCG, .cpp:2155-2226)
 __global__ void __launch_bounds__(128) k_mask_vec(DLevel L, float* v) {

@@ -16,7 +16,7 @@
 
 #include "common.cuh"
 #include "poisson_kernels.cuh"
-#include "staged_pipe.cuh"
+#include "poisson_march.cuh"
 
 namespace uaamg {
 
@@ -112,28 +112,20 @@ __device__ __forceinline__ float4 ldi4(const MLevel<T>& L, long long leaf, int t
     return f4scale(ldh4(L.invdiag, leaf, t), L.ics);
 }
 
-// storage and level traits of the pipelined staged kernels (staged_pipe.cuh)
+// storage and level traits of the marching sweeps (poisson_march.cuh)
 template <typename T>
 struct PipeE16 {
-    static constexpr unsigned ARR = UAAMG_LEAF * 2;
-    static __device__ __forceinline__ float4 s4(const unsigned char* a, int t) {
-        const uint2 u = reinterpret_cast<const uint2*>(a)[t];
-        const float2 p = H16<T>::to2(u.x), q = H16<T>::to2(u.y);
-        return make_float4(p.x, p.y, q.x, q.y);
+    static __device__ __forceinline__ float4 q(const T* p) { return ldh4(p, 0, 0); }
+    static __device__ __forceinline__ float v(const T* p) { return H16<T>::to1(*p); }
+    static __device__ __forceinline__ void st(T* p, float4 v) { sth4(p, 0, 0, v); }
+    static __device__ __forceinline__ void st2(T* p, float a, float b) {
+        *reinterpret_cast<unsigned*>(p) = H16<T>::from2(a, b);
     }
-    static __device__ __forceinline__ float s1(const unsigned char* a, int i) {
-        return H16<T>::bits1(reinterpret_cast<const unsigned short*>(a)[i]);
-    }
-    static __device__ __forceinline__ float bits1(unsigned short u) { return H16<T>::bits1(u); }
-    static __device__ __forceinline__ float4 g4(const T* p, long long leaf, int t) { return ldh4(p, leaf, t); }
-    static __device__ __forceinline__ float g1(const T* p, long long i) { return ldh1(p, i); }
-    static __device__ __forceinline__ void st(T* p, long long leaf, int t, float4 v) { sth4(p, leaf, t, v); }
-    static __device__ __forceinline__ void st1(T* p, long long i, float v) { p[i] = H16<T>::from1(v); }
 };
 template <> struct PipeE<__half> : PipeE16<__half> {};
 template <> struct PipeE<__nv_bfloat16> : PipeE16<__nv_bfloat16> {};
 template <typename T>
-struct PipeLv<MLevel<T>> {  // computes in stored units (staged_pipe.cuh)
+struct PipeLv<MLevel<T>> {  // computes in stored units (poisson_march.cuh)
     using E = T;
     static constexpr bool SCALED = true;
     static __device__ __forceinline__ float def_face(const MLevel<T>& L) { return __fmul_rn(L.def_face, L.ics); }
