@@ -16,6 +16,7 @@
 
 #include "viscosity_bottom.cuh"
 #include "viscosity_build.cuh"
+#include "viscosity_march.cuh"
 
 namespace {
 
@@ -272,6 +273,7 @@ struct VLevelDev {
     float* alt = nullptr;  // second buffer of the fused red-black steps (zero at non-DOF voxel groups), when used
     int* dof_base = nullptr;
     int* org = nullptr;
+    VPlain P{};  // the leaf lists, where the passes take plain leaves apart
 };
 
 }  // namespace
@@ -295,6 +297,9 @@ struct uaamg_viscosity {
     // (more leaves than resident CTAs: the next leaf's table loads hide behind
     // the current leaf)
     int seq_min_leaves = INT_MAX;
+    // levels of at least this many leaves take plain leaves apart in every pass (240^3, 2,491 leaves of level 1: 15.3
+    // to 13.0 us a colour; a 560-leaf level has 20 plain leaves and gains nothing)
+    int plain_min_leaves = 1024;
     std::vector<void*> allocs;
     // level-0 construction products kept for the right-hand side
     VolFields V{};
@@ -423,6 +428,26 @@ static void upload_defpage(uaamg_viscosity* h, VLevelDev& D) {
 static void upload_parents(uaamg_viscosity* h, const VHostLevel& H, VLevelDev& D) {
     D.L.parent = vupload(h, H.parent.data(), H.parent.size());
     D.L.octant = vupload(h, H.octant.data(), H.octant.size());
+}
+
+// The leaf lists of a level whose passes take plain leaves apart (viscosity_march.cuh).
+static void build_plain(uaamg_viscosity* h, VLevelDev& D) {
+    const int nl = D.L.nl;
+    if (nl < h->plain_min_leaves || nl <= h->rb_fused_max_leaves) return;
+    cudaStream_t s = h->stream;
+    int* list = (int*)valloc(h, (size_t)4 * nl * 4);
+    int* cnt = (int*)valloc(h, 16 * 4 + 27 * 4 + 4);
+    float* K = (float*)(cnt + 16);
+    int* cand = cnt + 16 + 27;
+    unsigned char* cls = (unsigned char*)valloc(h, (size_t)4 * nl);
+    uint32_t* carr = D.L.trim ? nullptr : (uint32_t*)valloc(h, (size_t)nl * 4);
+    if (!D.L.trim) {
+        CK(cudaMemsetAsync(cand, 0x7f, 4, s));
+        launch2(k_vconst, dim3((unsigned)nl), 128, s, D.L, carr, cand);
+    }
+    launch2(k_vclass, dim3((unsigned)((nl + 3) / 4)), 128, s, D.L, (const uint32_t*)carr, (const int*)cand, cls, K);
+    launch2(k_vlist, dim3(4), 1024, s, nl, (const unsigned char*)cls, list, cnt);
+    D.P = VPlain{list, cnt, K};
 }
 
 // k_vbottom's CG form by the coarsest system's size (rows per thread of a CTA of its own, 0: over eight CTAs)
@@ -673,6 +698,7 @@ static void build_viscosity(uaamg_viscosity* h, const uaamg_leaf_grid* mu_g, con
         h->C.slot = slot;
     }
     build_vbottom(h);
+    for (VLevelDev& D : h->lv) build_plain(h, D);
     // PCG vectors and scalars
     {
         const size_t vb = (size_t)3 * h->host[0].nl * UAAMG_LEAF * 4;
@@ -681,7 +707,7 @@ static void build_viscosity(uaamg_viscosity* h, const uaamg_leaf_grid* mu_g, con
             *v = (float*)valloc(h, vb);
             CK(cudaMemsetAsync(*v, 0, vb, s));
         }
-        size_t maxb = 1;
+        size_t maxb = (size_t)VMARCH_MINB * g_sms;  // CTAs of k_vmarch3
         for (auto& H : h->host) maxb = std::max(maxb, (size_t)3 * H.nl);
         h->partials = (double*)valloc(h, maxb * sizeof(double));
         h->st = (PcgState*)valloc(h, sizeof(PcgState) + 64);
@@ -718,7 +744,12 @@ struct VEnq {
         static const char* names[] = {"normal", "residual", "jacobi", "red_gs", "black_gs"};
         if (prof) pb("L" + std::to_string(l) + " " + names[MODE] + (gs ? " c" + std::to_string(c) : std::string()));
         if constexpr (MODE == VM_RED || MODE == VM_BLACK) {
-            if (D.L.nl >= h->seq_min_leaves) {
+            if (D.P.list) {
+                const dim3 g((unsigned)(VMARCH_MINB * g_sms));
+                if (c == 0) launch2(k_vmarch<MODE, 0>, g, VMARCH_THREADS, s, D.L, D.P, out, b, 1.0f);
+                else if (c == 1) launch2(k_vmarch<MODE, 1>, g, VMARCH_THREADS, s, D.L, D.P, out, b, 1.0f);
+                else launch2(k_vmarch<MODE, 2>, g, VMARCH_THREADS, s, D.L, D.P, out, b, 1.0f);
+            } else if (D.L.nl >= h->seq_min_leaves) {
                 const dim3 g((unsigned)std::min(D.L.nl, VAPPLY_MINB * g_sms));
                 if (c == 0) launch2(k_vapply_seq<MODE, 0>, g, 128, s, D.L, x, b, out, 1.0f);
                 else if (c == 1) launch2(k_vapply_seq<MODE, 1>, g, 128, s, D.L, x, b, out, 1.0f);
@@ -793,11 +824,20 @@ struct VEnq {
         pe();
         count++;
     }
+    template <int OP>
+    void march3(int l, const float* x, const float* b, VMarchOut O) {
+        const VLevelDev& D = h->lv[l];
+        const VLevel& C = OP == VM_RESTRICT ? h->lv[l + 1].L : D.L;
+        launch2(k_vmarch3<OP>, dim3((unsigned)(VMARCH_MINB * g_sms)), VMARCH_THREADS, s, D.L, C, D.P, x, b, O);
+    }
     // residual of level l restricted into the rhs of level l + 1 (fused); coarse_lhs (optional) is zeroed
     void residual_restrict(int l, const float* x, const float* b, float* coarse, float* coarse_lhs) {
         if (prof) pb("L" + std::to_string(l) + " residual+restrict");
-        launch2(k_vresrestrict, dim3((unsigned)h->lv[l].L.nl, 3), 128, s, h->lv[l].L, h->lv[l + 1].L, x, b, coarse,
-                coarse_lhs);
+        if (h->lv[l].P.list)
+            march3<VM_RESTRICT>(l, x, b, VMarchOut{coarse, coarse_lhs, nullptr, nullptr, 0, 0, 0});
+        else
+            launch2(k_vresrestrict, dim3((unsigned)h->lv[l].L.nl, 3), 128, s, h->lv[l].L, h->lv[l + 1].L, x, b, coarse,
+                    coarse_lhs);
         pe();
         count++;
     }
@@ -883,8 +923,11 @@ static void venqueue_setup(VEnq& E, cudaGraphConditionalHandle cond, int use_con
     launch2(k_vmask, g, 128, E.s, D.L, h->x);
     launch2(k_vmask, g, 128, E.s, D.L, h->b);
     if (E.prof) E.pb("L0 pcg init (residual+absmax)");
-    launch2(k_vpcg_init, g, 128, E.s, D.L, (const float*)h->x, (const float*)h->b, h->r, h->partials, h->st, cond,
-            use_cond);
+    if (D.P.list)
+        E.march3<VM_RESIDUAL>(0, h->x, h->b, VMarchOut{h->r, nullptr, h->partials, h->st, cond, use_cond, 0});
+    else
+        launch2(k_vpcg_init, g, 128, E.s, D.L, (const float*)h->x, (const float*)h->b, h->r, h->partials, h->st, cond,
+                use_cond);
     E.pe();
     E.count += 3;
 }
@@ -903,7 +946,8 @@ static void venqueue_body(VEnq& E, cudaGraphConditionalHandle cond, int use_cond
             (const PcgState*)h->st);
     E.pe();
     if (E.prof) E.pb("L0 pcg Ap");
-    launch2(k_vpcg_Ap, g, 128, E.s, D.L, (const float*)h->p, h->q);
+    if (D.P.list) E.march3<VM_NORMAL>(0, h->p, nullptr, VMarchOut{h->q, nullptr, nullptr, nullptr, 0, 0, 0});
+    else launch2(k_vpcg_Ap, g, 128, E.s, D.L, (const float*)h->p, h->q);
     E.pe();
     if (E.prof) E.pb("L0 pcg sigma (p.q)");
     launch2(k_vdot, gd, VDOT_THREADS, E.s, D.L, (const float*)h->p, (const float*)h->q, part, h->st, 1);
@@ -1203,6 +1247,7 @@ int uaamg_viscosity_create_on_stream(const uaamg_leaf_grid* viscosity, const uaa
         h->seq_min_leaves = 2 * g_sms + 1;
         if (const char* e = getenv("UAAMG_VISC_FUSED_RB_LEAVES")) h->rb_fused_max_leaves = atoi(e);
         if (const char* e = getenv("UAAMG_VISC_SEQ_LEAVES")) h->seq_min_leaves = atoi(e);
+        if (const char* e = getenv("UAAMG_VISC_PLAIN_LEAVES")) h->plain_min_leaves = atoi(e);
         build_viscosity(h, viscosity, liquid_sdf, solid_sdf, dt, rho, dx);
     } catch (const UaamgError& e) {
         uaamg_viscosity_destroy(h);

@@ -405,24 +405,33 @@ __device__ __forceinline__ float4 vapply_value(const VLevel& L, const VNbSh& sh,
     return res;
 }
 
-// One applier pass over one leaf and channel c (a constant); m = DOF bits.
+// One applier pass over one leaf and channel c (a constant), returning the
+// thread's values (0 where it has no DOF).
 // Static data first (DOF mask, neighbourhood, coefficients): they are not
 // written during a solve, so they load while the previous kernel is still
 // running; the vectors are read after griddepcontrol.wait.
-template <int MODE, int c>
-__device__ __forceinline__ void vapply_leaf(const VLevel& L, VNbSh& sh, int leaf, const float* x, const float* b,
-                                            float* out, float w) {
+template <int MODE, int c, bool WAIT = true>
+__device__ __forceinline__ float4 vapply_tab(const VLevel& L, const VNbSh& sh, int leaf, unsigned m, const float* x,
+                                             const float* b, float* out, float w) {
     const int t = threadIdx.x;
-    const unsigned m = vmask4(L, c, leaf, t);
-    vnb_prologue(L, leaf, sh);
     VCoef k;
     if (m) vload_coef<MODE, c>(L, sh, t, k);
-    griddep_wait();
-    griddep_launch();
-    if (!m) return;
+    if (WAIT) {
+        griddep_wait();
+        griddep_launch();
+    }
+    if (!m) return f4zero();
     float4 xc;
     const float4 res = vapply_value_k<MODE, c>(L, sh, t, x, b, w, m, k, xc);
     reinterpret_cast<float4*>(out + (long long)c * L.nl * UAAMG_LEAF)[(long long)leaf * UAAMG_LEAF4 + t] = res;
+    return res;
+}
+template <int MODE, int c>
+__device__ __forceinline__ float4 vapply_leaf(const VLevel& L, VNbSh& sh, int leaf, const float* x, const float* b,
+                                              float* out, float w) {
+    const unsigned m = vmask4(L, c, leaf, threadIdx.x);
+    vnb_prologue(L, leaf, sh);
+    return vapply_tab<MODE, c>(L, sh, leaf, m, x, b, out, w);
 }
 
 #ifndef VAPPLY_MINB
@@ -837,36 +846,44 @@ __global__ void __launch_bounds__(128) k_vrestrict(VLevel F, VLevel C, const flo
 // summation order as k_vapply<VM_RESIDUAL> + k_vrestrict; the coarse voxels of
 // octants without a fine leaf are never written (they hold no DOF, and the
 // coarse rhs is zero there from allocation).
-template <int c>
-__device__ __forceinline__ void vresrestrict_leaf(const VLevel& F, const VLevel& C, VNbSh& sh, float* rs, int leaf,
-                                                  const float* x, const float* b, float* coarse, float* coarse_lhs) {
+template <int c, bool WAIT = true>
+__device__ __forceinline__ void vresrestrict_tab(const VLevel& F, const VLevel& C, const VNbSh& sh, float* rs, int leaf,
+                                                 unsigned m, const float* x, const float* b, float* coarse,
+                                                 float* coarse_lhs) {
     const int t = threadIdx.x;
-    const unsigned m = vmask4(F, c, leaf, t);
-    vnb_prologue(F, leaf, sh);
     VCoef k;
     if (m) vload_coef<VM_RESIDUAL, c>(F, sh, t, k);
     // static: parent, octant, the DOF mask words of this thread's coarse
     // voxel (t < 64: one of the 4x4x4 coarse voxels of the octant)
-    const int P = F.parent[leaf];
-    const int oc = F.octant[leaf];
+    int P = -1, cx = 0, cy = 0, cz = 0;
     const int ci = t >> 4, cj = (t >> 2) & 3, ck = t & 3;
-    const int cx = ((oc >> 2) & 1) * 4 + ci, cy = ((oc >> 1) & 1) * 4 + cj, cz = (oc & 1) * 4 + ck;
     bool cdof = false;
     uint64_t fw[2] = {0ull, 0ull};
-    if (t < 64 && P >= 0) {
-        cdof = vdof_bit(C, c, P, voff3(cx, cy, cz));
-        const uint64_t* fm = F.dof + ((long long)c * F.nl + leaf) * 8;
-        fw[0] = fm[2 * ci];
-        fw[1] = fm[2 * ci + 1];
+    auto place = [&] {
+        P = F.parent[leaf];
+        const int oc = F.octant[leaf];
+        cx = ((oc >> 2) & 1) * 4 + ci;
+        cy = ((oc >> 1) & 1) * 4 + cj;
+        cz = (oc & 1) * 4 + ck;
+        if (t < 64 && P >= 0) {
+            cdof = vdof_bit(C, c, P, voff3(cx, cy, cz));
+            const uint64_t* fm = F.dof + ((long long)c * F.nl + leaf) * 8;
+            fw[0] = fm[2 * ci];
+            fw[1] = fm[2 * ci + 1];
+        }
+    };
+    if (WAIT) {  // with the coefficients, while the previous kernel runs
+        place();
+        griddep_wait();
+        griddep_launch();
     }
-    griddep_wait();
-    griddep_launch();
     float4 res = f4zero();
     if (m) {
         float4 xc;
         res = vapply_value_k<VM_RESIDUAL, c>(F, sh, t, x, b, 1.f, m, k, xc);
     }
     reinterpret_cast<float4*>(rs)[t] = res;
+    if (!WAIT) place();
     __syncthreads();
     if (t < 64 && P >= 0) {
         float s = 0.f;
@@ -888,6 +905,13 @@ __device__ __forceinline__ void vresrestrict_leaf(const VLevel& F, const VLevel&
         // fine leaf has a DOF of c, so these writes cover them (the memset they replace was a graph node of its own)
         if (coarse_lhs) coarse_lhs[((long long)c * C.nl + P) * UAAMG_LEAF + voff3(cx, cy, cz)] = 0.f;
     }
+}
+template <int c>
+__device__ __forceinline__ void vresrestrict_leaf(const VLevel& F, const VLevel& C, VNbSh& sh, float* rs, int leaf,
+                                                  const float* x, const float* b, float* coarse, float* coarse_lhs) {
+    const unsigned m = vmask4(F, c, leaf, threadIdx.x);
+    vnb_prologue(F, leaf, sh);
+    vresrestrict_tab<c>(F, C, sh, rs, leaf, m, x, b, coarse, coarse_lhs);
 }
 __global__ void __launch_bounds__(128, VAPPLY_MINB) k_vresrestrict(VLevel F, VLevel C, const float* x, const float* b,
                                                                    float* coarse, float* coarse_lhs) {
@@ -987,6 +1011,21 @@ __device__ __forceinline__ float vabs4(float4 v, unsigned m) {
     return a;
 }
 
+__device__ __forceinline__ void vpcg_start(PcgState* st, float nu, cudaGraphConditionalHandle cond, int use_cond) {
+    st->nu = nu;
+    st->numax = __fmul_rn(st->tol, nu);
+    st->iter = 0;
+    st->first = 1;
+    st->iterations_taken = 0;
+    st->alpha = 0.f;
+    st->beta = 0.f;
+    int status = PCG_RUNNING;
+    if (nu <= st->numax) status = PCG_SUCCESS;
+    else if (st->max_iter <= 0) status = PCG_FAILED_MAXITER;  // loop never runs: x untouched
+    st->status = status;
+    st->ticket[1] = 0;
+    set_cond(cond, use_cond, status == PCG_RUNNING ? 1u : 0u);
+}
 // lines 2-3: r = b - A x; nu = |r|_inf; numax = tol * nu
 __global__ void __launch_bounds__(128) k_vpcg_init(VLevel L, const float* x, const float* b, float* r,
                                                    double* partials, PcgState* st, cudaGraphConditionalHandle cond,
@@ -1009,21 +1048,7 @@ __global__ void __launch_bounds__(128) k_vpcg_init(VLevel L, const float* x, con
     const float part = block_max128(a, shf);
     if (vpublish((double)part, partials, &st->ticket[1], &last)) {
         const float nu = vgather_max(partials, shf);
-        if (t == 0) {
-            st->nu = nu;
-            st->numax = __fmul_rn(st->tol, nu);
-            st->iter = 0;
-            st->first = 1;
-            st->iterations_taken = 0;
-            st->alpha = 0.f;
-            st->beta = 0.f;
-            int status = PCG_RUNNING;
-            if (nu <= st->numax) status = PCG_SUCCESS;
-            else if (st->max_iter <= 0) status = PCG_FAILED_MAXITER;  // loop never runs: x untouched
-            st->status = status;
-            st->ticket[1] = 0;
-            set_cond(cond, use_cond, status == PCG_RUNNING ? 1u : 0u);
-        }
+        if (t == 0) vpcg_start(st, nu, cond, use_cond);
     }
 }
 
