@@ -21,7 +21,6 @@
 // kernels, and each reduction keeps the instance's leaf slots and order, so
 // each instance's result, iteration count and status are bit-identical to its
 // standalone solve.
-#include <array>
 
 namespace {
 
@@ -115,7 +114,49 @@ __global__ void __launch_bounds__(128, 7) k_brestrict(const BRec* __restrict__ r
     restrict_leaf<true, true>(R.L, e.y, R.v[xr], R.v[br], R.v[BR_CRHS], active + e.x);
 }
 
-template <int ROWS, int NT>
+// The passes of k_bsweep / k_brestrict as marching sweeps (poisson_march.cuh):
+// eight pairs of planes per CTA, whatever instances they belong to.  Plain
+// sources without a dot product; values are those of the kernels above.
+constexpr int BMARCH_NP = 2;
+template <int MODE, bool RESTRICT>
+__global__ void __launch_bounds__(MARCH_THREADS, MARCH_MINB) k_bmarch(const BRec* __restrict__ recs,
+                                                                      const int2* __restrict__ map, int count,
+                                                                      const unsigned* active, int xr, int br, int outr,
+                                                                      float w) {
+    constexpr int SEG = 8 / BMARCH_NP;
+    const long long item = (long long)blockIdx.x * (MARCH_THREADS / 16) + (threadIdx.x >> 4);
+    const bool on = item < (long long)count * SEG;
+    const int2 e = map[on ? (int)(item / SEG) : count - 1];
+    const BRec& R = recs[e.x];
+    const float ws = R.w_sor;
+    march_leaf<MODE, DLevel, float, RESTRICT, BMARCH_NP>(R.L, e.y, (int)(item % SEG) * BMARCH_NP, on, R.v[xr], R.v[br],
+                                                         R.v[outr], w, ws, 1.0f - ws, DotOut{nullptr, nullptr, nullptr},
+                                                         nullptr, 0.f, active + e.x);
+}
+// The value of a source stored (k_materialize); into x itself for a prolongation.
+template <int SRC>
+__global__ void __launch_bounds__(128) k_bmaterialize(const BRec* __restrict__ recs, const int2* __restrict__ map,
+                                                      const unsigned* active, int xr, int br, int outr, float wsrc) {
+    const int2 e = map[blockIdx.x];
+    const BRec& R = recs[e.x];
+    const int t = threadIdx.x;
+    const unsigned m = mask4(R.L.mask, e.y, t);
+    griddep_wait();
+    griddep_launch();
+    if (!active[e.x]) return;
+    float4 v;
+    if (SRC == S_FIRST_JACOBI) v = SrcFirstJacobi{R.v[br], wsrc}.get4(R.L, e.y, t);
+    else v = SrcProlong{R.v[xr], R.v[BR_CLHS], 1.0f}.get4(R.L, e.y, t);
+    if (!(m & 1)) v.x = 0.f;
+    if (!(m & 2)) v.y = 0.f;
+    if (!(m & 4)) v.z = 0.f;
+    if (!(m & 8)) v.w = 0.f;
+    st4(R.v[outr], e.y, t, v);
+}
+
+// Coarsest solves, a CTA per instance of any size class.  (A launch per class
+// left the few CTAs of one waiting for those of another: 40 instances of 32^3 to
+// 192^3, the launches of the three classes at a depth, 15 + 19 + 32 us in turn.)
 __global__ void __launch_bounds__(CG_THREADS, 1) k_bcoarsest(const BRec* __restrict__ recs, const int* __restrict__ list,
                                                      const unsigned* __restrict__ active, int br, int outr) {
     griddep_wait();
@@ -125,7 +166,11 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_bcoarsest(const BRec* __restr
     const int i = list[blockIdx.x];
     if (!active[i]) return;
     const BRec& R = recs[i];
-    coarsest_cg_body<ROWS, NT, false>(R.C, R.v[br], R.v[outr], cg_ps, red);
+    switch (coarsest_class(R.C.n)) {
+    case 0: coarsest_cg_body<2, 512, false>(R.C, R.v[br], R.v[outr], cg_ps, red); break;
+    case 1: coarsest_cg_body<4, 512, false>(R.C, R.v[br], R.v[outr], cg_ps, red); break;
+    default: coarsest_cg_body<4, 1024, false>(R.C, R.v[br], R.v[outr], cg_ps, red);
+    }
 }
 
 __global__ void __launch_bounds__(128) k_bdot_rho(const BRec* __restrict__ recs, const int2* __restrict__ map,
@@ -265,7 +310,8 @@ struct uaamg_batch {
     };
     Range all0, dot1;
     std::vector<Range> smooth;                  // [depth]
-    std::vector<std::array<Range, 3>> coarse;   // [depth][ROWS 1, 2, 4]
+    std::vector<Range> coarse;                  // [depth]
+    std::vector<unsigned> coarse_smem;          // [depth] shared memory of its largest coarsest system
     // graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -278,6 +324,13 @@ struct uaamg_batch {
 
 namespace {
 
+// Depths of at least this many leaves over all instances march, and store the
+// first sweep's source and the prolongation first.  40 instances of 32^3 to
+// 192^3, k_bsweep / march with a cold L2: 14,420 leaves 71 / 39 us (a first sweep
+// 74 / 59 with its store, after prolongation 95 / 59, restriction 61 / 35),
+// 2,578 leaves 17.8 / 13.7.  A depth of 405 leaves takes 8.6 us a sweep either way,
+// and the store would add launches.
+#define BMARCH_MIN_LEAVES 1024
 struct BEnq {
     uaamg_batch* b;
     cudaStream_t s;
@@ -286,33 +339,50 @@ struct BEnq {
     const int2* map(const uaamg_batch::Range& r) const { return b->maps + r.off; }
     bool smooths(int d) const { return d < (int)b->smooth.size() && b->smooth[d].count > 0; }
 
+    // depths that march, and whose computed sources are stored first (T: the buffer for them)
+    bool marches(int d) const { return b->smooth[d].count >= BMARCH_MIN_LEAVES; }
     template <int MODE, int SRC>
     void sweep(int d, int xr, int br, int outr, float w, float wsrc = 0.f, int dot = 0, int mark = 0) {
         const uaamg_batch::Range& r = b->smooth[d];
-        launch(k_bsweep<MODE, SRC>, (unsigned)r.count, 128, s, recs(d), map(r), (const unsigned*)b->active, xr, br,
-               outr, w, wsrc, dot, mark);
+        const unsigned* act = b->active;
+        if constexpr (MODE == M_JACOBI && (SRC == S_FIRST_JACOBI || SRC == S_PROLONG)) {
+            if (marches(d)) {
+                launch(k_bmaterialize<SRC>, (unsigned)r.count, 128, s, recs(d), map(r), act, xr, br, (int)BR_TMP, wsrc);
+                count++;
+                sweep<MODE, S_PLAIN>(d, BR_TMP, br, outr, w, 0.f, dot, mark);
+                return;
+            }
+        }
+        if constexpr (SRC == S_PLAIN) {
+            if (marches(d) && !dot && !mark) {
+                launch(k_bmarch<MODE, false>, march_grid(r.count, BMARCH_NP), MARCH_THREADS, s, recs(d), map(r),
+                       r.count, act, xr, br, outr, w);
+                count++;
+                return;
+            }
+        }
+        launch(k_bsweep<MODE, SRC>, (unsigned)r.count, 128, s, recs(d), map(r), act, xr, br, outr, w, wsrc, dot, mark);
         count++;
     }
     void restrict_resid(int d, int xr, int br) {
         const uaamg_batch::Range& r = b->smooth[d];
-        launch(k_brestrict, (unsigned)r.count, 128, s, recs(d), map(r), (const unsigned*)b->active, xr, br);
+        const unsigned* act = b->active;
+        if (marches(d))
+            launch(k_bmarch<M_RESIDUAL, true>, march_grid(r.count, BMARCH_NP), MARCH_THREADS, s, recs(d), map(r),
+                   r.count, act, xr, br, (int)BR_CRHS, 0.f);
+        else
+            launch(k_brestrict, (unsigned)r.count, 128, s, recs(d), map(r), act, xr, br);
         count++;
     }
-    // coarsest solves of the instances whose hierarchy ends at depth d (rows
-    // per thread as in the single solve), then z.r for one-level hierarchies
+    // coarsest solves of the instances whose hierarchy ends at depth d, then z.r for one-level hierarchies
     void coarsest(int d, int br, int outr, bool dot) {
-        const std::array<uaamg_batch::Range, 3>& c = b->coarse[d];
+        const uaamg_batch::Range& c = b->coarse[d];
         const unsigned* act = b->active;
-        if (c[0].count)
-            launch_smem(k_bcoarsest<2, 512>, (unsigned)c[0].count, CG_THREADS, cg_smem_bytes<2, 512>(), s, recs(d),
-                        b->lists + c[0].off, act, br, outr);
-        if (c[1].count)
-            launch_smem(k_bcoarsest<4, 512>, (unsigned)c[1].count, CG_THREADS, cg_smem_bytes<4, 512>(), s, recs(d),
-                        b->lists + c[1].off, act, br, outr);
-        if (c[2].count)
-            launch_smem(k_bcoarsest<4, 1024>, (unsigned)c[2].count, CG_THREADS, cg_smem_bytes<4, 1024>(), s, recs(d),
-                        b->lists + c[2].off, act, br, outr);
-        count += (c[0].count > 0) + (c[1].count > 0) + (c[2].count > 0);
+        if (c.count) {
+            launch_smem(k_bcoarsest, (unsigned)c.count, CG_THREADS, b->coarse_smem[d], s, recs(d), b->lists + c.off, act,
+                        br, outr);
+            count++;
+        }
         if (dot && d == 0 && b->dot1.count) {
             launch(k_bdot_rho, (unsigned)b->dot1.count, 128, s, recs(0), map(b->dot1), act);
             count++;
@@ -520,23 +590,25 @@ static void bbuild_tables(uaamg_batch* b) {
     add_map([](uaamg_poisson*) { return true; }, b->all0, [](uaamg_poisson*) { return 0; });
     add_map([](uaamg_poisson* h) { return h->nlev == 1; }, b->dot1, [](uaamg_poisson*) { return 0; });
     b->smooth.assign(b->depth, uaamg_batch::Range());
-    b->coarse.assign(b->depth, std::array<uaamg_batch::Range, 3>());
+    b->coarse.assign(b->depth, uaamg_batch::Range());
+    b->coarse_smem.assign(b->depth, 0);
     for (int d = 0; d < b->depth; ++d) {
         add_map([d](uaamg_poisson* h) { return h->nlev - 1 > d; }, b->smooth[d], [d](uaamg_poisson*) { return d; });
-        for (int k = 0; k < 3; ++k) {
-            uaamg_batch::Range& r = b->coarse[d][k];
-            r.off = (int)lists.size();
-            for (int i = 0; i < n; ++i) {
-                uaamg_poisson* h = b->inst[i];
-                if (h->lv.empty() || h->lv[0].L.nl == 0 || h->nlev - 1 != d || h->C.n == 0) continue;
-                const int cls = coarsest_class(h->C.n);
-                if (cls == k) lists.push_back(i);
-            }
-            r.count = (int)lists.size() - r.off;
+        uaamg_batch::Range& r = b->coarse[d];
+        r.off = (int)lists.size();
+        for (int i = 0; i < n; ++i) {
+            uaamg_poisson* h = b->inst[i];
+            if (h->lv.empty() || h->lv[0].L.nl == 0 || h->nlev - 1 != d || h->C.n == 0) continue;
+            const int cls = coarsest_class(h->C.n);
+            const unsigned smem = cls == 0   ? cg_smem_bytes<2, 512>()
+                                  : cls == 1 ? cg_smem_bytes<4, 512>()
+                                             : cg_smem_bytes<4, 1024>();
+            b->coarse_smem[d] = std::max(b->coarse_smem[d], smem);
+            lists.push_back(i);
         }
+        r.count = (int)lists.size() - r.off;
     }
-    CK(cudaFuncSetAttribute(k_bcoarsest<4, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            cg_smem_bytes<4, 1024>()));
+    CK(cudaFuncSetAttribute(k_bcoarsest, cudaFuncAttributeMaxDynamicSharedMemorySize, cg_smem_bytes<4, 1024>()));
     // one device allocation: records, maps, lists, active flags, pointer
     // arrays, global counters, gathered states
     const size_t nrec = (size_t)b->depth * n;

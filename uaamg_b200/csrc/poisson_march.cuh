@@ -128,26 +128,24 @@ __host__ __device__ __forceinline__ unsigned march_grid(int nl, int NP) {
     return (unsigned)(((long long)nl * (8 / NP) + 7) / 8);
 }
 
-// One sweep (RESTRICT false: out[leaf] = value, optionally scaled by *zscale
-// and with a fused dot) or one residual + restriction (RESTRICT true, MODE
-// M_RESIDUAL: coarse = 0.125 * sum of the active fine residuals of each 2x2x2
-// block, times coarse_scale on 16-bit levels) over a level.  RED and BLACK may
-// run in place: what an update reads of its own colour is its own voxel.
-// DOTK: 0 z.r with the b of a level-0 sweep or dot.r (PCG lines 13-15: rho,
-// beta), 1 p.q with p the swept vector (the Laplacian of PCG lines 6-7: sigma,
-// alpha); a partial per CTA, in an order that depends on the level only.
+// NP planes from X0 on of a leaf, by the 16 lanes q of a half-warp: a sweep
+// (RESTRICT false: out[leaf] = value, optionally scaled by *zscale; returns the
+// lane's part of the dot product, if dot.r) or residual + restriction (RESTRICT
+// true, MODE M_RESIDUAL: coarse = 0.125 * sum of the active fine residuals of
+// each 2x2x2 block, times coarse_scale on 16-bit levels).  RED and BLACK may run
+// in place: what an update reads of its own colour is its own voxel.  on: the
+// half-warp has a leaf (else it follows the other half); gate: nothing is
+// written if this word is zero.  DOTK: 0 z.r with the b of a level-0 sweep or
+// dot.r, 1 p.q with p the swept vector.
 template <int MODE, class LV, typename TOut, bool RESTRICT, int NP, int DOTK = 0>
-__global__ void __launch_bounds__(MARCH_THREADS, PipeLv<LV>::SCALED ? MARCH_MINB16 : MARCH_MINB)
-    k_march(LV L, const typename PipeLv<LV>::E* x, const typename PipeLv<LV>::E* b, TOut* out, float w, float wsor,
-            float one_minus_wsor, DotOut dot, const float* zscale, float coarse_scale) {
+__device__ __forceinline__ double march_leaf(const LV& L, int leaf, int X0, bool on,
+                                             const typename PipeLv<LV>::E* x, const typename PipeLv<LV>::E* b, TOut* out,
+                                             float w, float wsor, float one_minus_wsor, const DotOut& dot,
+                                             const float* zscale, float coarse_scale, const unsigned* gate = nullptr) {
     using T = PipeLv<LV>;
     using E = typename T::E;
     using P = PipeE<E>;
-    constexpr int SEG = 8 / NP;
-    const int lane = threadIdx.x & 31, half = lane >> 4, q = lane & 15, Y = q >> 1, zh = q & 1;
-    const long long item = ((long long)blockIdx.x * (MARCH_THREADS / 32) + (threadIdx.x >> 5)) * 2 + half;
-    const bool on = item < (long long)L.nl * SEG;
-    const int leaf = on ? (int)(item / SEG) : L.nl - 1, X0 = (int)(item % SEG) * NP;
+    const int lane = threadIdx.x & 31, q = lane & 15, Y = q >> 1, zh = q & 1;
     const long long l0 = (long long)leaf * UAAMG_LEAF;
     // ---- static data, before the wait for the previous kernel
     const int2* nbp = reinterpret_cast<const int2*>(L.nbr + (long long)leaf * 6);
@@ -179,6 +177,10 @@ __global__ void __launch_bounds__(MARCH_THREADS, PipeLv<LV>::SCALED ? MARCH_MINB
     else div = T::def_invdiag(L);
     griddep_wait();
     griddep_launch();
+    if (gate) {
+        on = on && *gate != 0;
+        if (!__any_sync(FULLMASK, on)) return 0.0;
+    }
 
     auto plane = [&](int i) {
         MarchPlane r;
@@ -314,6 +316,22 @@ __global__ void __launch_bounds__(MARCH_THREADS, PipeLv<LV>::SCALED ? MARCH_MINB
             A = B;
         }
     }
+    return sum;
+}
+
+// One pass over a level (march_leaf).  The dot products: rho and beta (PCG lines
+// 13-15, DOTK 0), or sigma and alpha (lines 6-7, DOTK 1); a partial per CTA, in
+// an order that depends on the level only.
+template <int MODE, class LV, typename TOut, bool RESTRICT, int NP, int DOTK = 0>
+__global__ void __launch_bounds__(MARCH_THREADS, PipeLv<LV>::SCALED ? MARCH_MINB16 : MARCH_MINB)
+    k_march(LV L, const typename PipeLv<LV>::E* x, const typename PipeLv<LV>::E* b, TOut* out, float w, float wsor,
+            float one_minus_wsor, DotOut dot, const float* zscale, float coarse_scale) {
+    constexpr int SEG = 8 / NP;
+    const long long item = (long long)blockIdx.x * (MARCH_THREADS / 16) + (threadIdx.x >> 4);
+    const bool on = item < (long long)L.nl * SEG;
+    const int leaf = on ? (int)(item / SEG) : L.nl - 1, X0 = (int)(item % SEG) * NP;
+    const double sum = march_leaf<MODE, LV, TOut, RESTRICT, NP, DOTK>(L, leaf, X0, on, x, b, out, w, wsor, one_minus_wsor,
+                                                                       dot, zscale, coarse_scale);
     if constexpr (!RESTRICT) {
         if (dot.r) {
             __shared__ double shd[MARCH_THREADS / 32];
