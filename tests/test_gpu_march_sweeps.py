@@ -94,3 +94,24 @@ def test_mixed_solve_equal(tuned, n, precision):
         got.append((p, status, s.mIterationTaken))
     assert got[0][1:] == got[1][1:]
     assert np.array_equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("smoother", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [104, 131])
+def test_solve_equal(tuned, n, smoother):
+    """Level 0 of 1,024 to 8,191 leaves: the passes with dot products march too,
+    with the one-leaf kernels' sums, so a whole solve is equal."""
+    from uaamg_b200.poisson import PoissonSolver
+    sc = scenes.large_poisson_scene(n=n, seed=4)
+    got = []
+    for staged in (64, NEVER):
+        tuned({"staged_min_leaves": staged})
+        lap = laplacian(sc)
+        assert 1024 <= lap.leaf_count(0) < 8192
+        rhs = lap.createPressurePoissonRightHandSide(sc.face_weights, sc.vx, sc.vy, sc.vz, sc.solid_velocity, sc.dt)
+        s = PoissonSolver(lap)
+        s.mSmoother = PoissonSolver.SmootherOption(smoother)
+        p = lap.getZeroVectorGrid()
+        got.append((p, s.solveMultigridPCG(p, rhs), s.mIterationTaken))
+    assert got[0][1:] == got[1][1:]
+    assert np.array_equal(got[0][0], got[1][0])

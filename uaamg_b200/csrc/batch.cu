@@ -133,6 +133,23 @@ __global__ void __launch_bounds__(MARCH_THREADS, MARCH_MINB) k_bmarch(const BRec
                                                          R.v[outr], w, ws, 1.0f - ws, DotOut{nullptr, nullptr, nullptr},
                                                          nullptr, 0.f, active + e.x);
 }
+// A sweep with z.r (DOTK 0), or A p with p.q (DOTK 1): a leaf per CTA, a plane per
+// half-warp, so that each thread holds the voxels that the one-leaf kernels'
+// threads hold and the sums are theirs.
+template <int MODE, int DOTK>
+__global__ void __launch_bounds__(MARCH_THREADS, MARCH_MINB) k_bmarch_dot(const BRec* __restrict__ recs,
+                                                                          const int2* __restrict__ map,
+                                                                          const unsigned* active, int xr, int br, int outr,
+                                                                          float w) {
+    const int2 e = map[blockIdx.x];
+    const BRec& R = recs[e.x];
+    const float ws = R.w_sor;
+    const DotOut d{R.v[DOTK == 1 ? xr : BR_R], R.partials, R.st};
+    const double sum = march_leaf<MODE, DLevel, float, false, 1, DOTK>(R.L, e.y, threadIdx.x >> 4, true, R.v[xr], R.v[br],
+                                                                       R.v[outr], w, ws, 1.0f - ws, d, nullptr, 0.f,
+                                                                       active + e.x);
+    if (active[e.x]) march_dot<DOTK>(sum, d, e.y, R.L.nl);
+}
 // The value of a source stored (k_materialize); into x itself for a prolongation.
 template <int SRC>
 __global__ void __launch_bounds__(128) k_bmaterialize(const BRec* __restrict__ recs, const int2* __restrict__ map,
@@ -354,7 +371,12 @@ struct BEnq {
             }
         }
         if constexpr (SRC == S_PLAIN) {
-            if (marches(d) && !dot && !mark) {
+            if (marches(d) && dot && !mark) {
+                launch(k_bmarch_dot<MODE, 0>, (unsigned)r.count, MARCH_THREADS, s, recs(d), map(r), act, xr, br, outr, w);
+                count++;
+                return;
+            }
+            if (marches(d) && !mark) {
                 launch(k_bmarch<MODE, false>, march_grid(r.count, BMARCH_NP), MARCH_THREADS, s, recs(d), map(r),
                        r.count, act, xr, br, outr, w);
                 count++;
@@ -468,7 +490,11 @@ static void benqueue_body(BEnq& E, cudaGraphConditionalHandle cond, int use_cond
     benqueue_precond(E, 0, BR_Z, BR_R, true, true);
     const unsigned g0 = (unsigned)b->all0.count;
     launch(k_bpcg_update_p, g0, 128, E.s, E.recs(0), E.map(b->all0), (const unsigned*)b->active);
-    launch(k_bpcg_Ap, g0, 128, E.s, E.recs(0), E.map(b->all0), (const unsigned*)b->active);
+    if (b->all0.count >= BMARCH_MIN_LEAVES)
+        launch(k_bmarch_dot<M_LAPLACIAN, 1>, g0, MARCH_THREADS, E.s, E.recs(0), E.map(b->all0), (const unsigned*)b->active,
+               (int)BR_P, (int)BR_R, (int)BR_Q, 0.f);
+    else
+        launch(k_bpcg_Ap, g0, 128, E.s, E.recs(0), E.map(b->all0), (const unsigned*)b->active);
     launch(k_bpcg_update_r, g0, 128, E.s, E.recs(0), E.map(b->all0), b->n, b->active, b->g, cond, use_cond);
     E.count += 3;
 }

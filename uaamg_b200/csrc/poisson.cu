@@ -1036,9 +1036,15 @@ static int g_sms = 148;  // SMs of the device (set when a handle is created)
 // 187 / 177; 16-bit sweep at 30,492: 54 / 49.
 static int march_planes(int nl, bool fp32_sweep = false) { return nl >= (fp32_sweep ? 65536 : 24576) ? 8 : 2; }
 // A pass that carries a level-0 dot product (the last post-smoothing sweep
-// with z.r, A p with p.q) marches from this fixed size on: its per-CTA
-// partials set the dot's summation order, which must not depend on the tuning.
+// with z.r, A p with p.q) marches two or eight planes from PIPE_DOT_MIN_LEAVES
+// leaves on: its per-CTA partials set the dot's summation order, which must not
+// depend on the tuning.  Below, from DOT_MARCH_MIN_LEAVES on, a leaf per CTA
+// and a plane per half-warp: a thread then holds the voxels it holds in the
+// one-leaf kernels and the sums are theirs (6,400 leaves, one-leaf / marching:
+// A p 21 / 19 us, sweep 21 / 19; 1,916 leaves: 16.8 / 14.8, 16.8 / 16.8).  The
+// mixed-precision form marches its dot from PIPE_DOT_MIN_LEAVES on.
 #define PIPE_DOT_MIN_LEAVES 8192
+#define DOT_MARCH_MIN_LEAVES 1024
 // Grid of the grid-stride elementwise kernels (k_materialize, the PCG
 // vector updates): 16 CTAs of 128 threads per SM of a 148-SM B200, at most
 // one per leaf.  One CTA per leaf would make a large level's elementwise
@@ -1244,13 +1250,14 @@ struct Enq {
         if constexpr (std::is_same<Src, SrcPlain>::value) {
             if (g_use_staged && D.L.nl >= STAGED_MIN_LEAVES && !(MODE == M_SPAI0 && mark_spai0)) {
                 if (prof) pb("L" + std::to_string(l) + " " + mode_name(MODE) + " staged" + (dot.r ? "+dot" : ""));
-                if (D.L.nl >= (dot.r ? PIPE_DOT_MIN_LEAVES : PIPE_MIN_LEAVES)) {
+                if (D.L.nl >= (dot.r ? DOT_MARCH_MIN_LEAVES : PIPE_MIN_LEAVES)) {
                     auto go = [&](auto kern, int NP) {
                         launch_march(kern, D.L.nl, NP, s, D.L, (const float*)src.x, b, out, w, ws, 1.0f - ws, dot,
                                      (const float*)nullptr, 0.f);
                     };
                     const int NP = march_planes(D.L.nl, !dot.r);
-                    if (NP == 8) go(k_march<MODE, DLevel, float, false, 8>, 8);
+                    if (dot.r && D.L.nl < PIPE_DOT_MIN_LEAVES) go(k_march<MODE, DLevel, float, false, 1>, 1);
+                    else if (NP == 8) go(k_march<MODE, DLevel, float, false, 8>, 8);
                     else go(k_march<MODE, DLevel, float, false, 2>, 2);
                 } else
                     launch(k_sweep_staged<MODE>, (unsigned)D.L.nl, 128, s, D.L, (const float*)src.x, b, out, w, ws,
@@ -1606,10 +1613,12 @@ static void enqueue_setup(Enq& E, cudaGraphConditionalHandle cond, int use_cond)
 static void enqueue_Ap(Enq& E) {
     uaamg_poisson* h = E.h;
     LevelDev& D0 = h->lv[0];
-    if (g_use_staged && D0.L.nl >= PIPE_DOT_MIN_LEAVES) {
-        const int NP = march_planes(D0.L.nl);
-        launch_march(NP == 8 ? k_march<M_LAPLACIAN, DLevel, float, false, 8, 1>
-                             : k_march<M_LAPLACIAN, DLevel, float, false, 2, 1>,
+    const bool large = D0.L.nl >= PIPE_DOT_MIN_LEAVES;
+    if (g_use_staged && (large || D0.L.nl >= std::max(DOT_MARCH_MIN_LEAVES, (int)STAGED_MIN_LEAVES))) {
+        const int NP = large ? march_planes(D0.L.nl) : 1;
+        launch_march(NP == 8   ? k_march<M_LAPLACIAN, DLevel, float, false, 8, 1>
+                     : NP == 2 ? k_march<M_LAPLACIAN, DLevel, float, false, 2, 1>
+                               : k_march<M_LAPLACIAN, DLevel, float, false, 1, 1>,
                      D0.L.nl, NP, E.s, D0.L, (const float*)h->p, (const float*)nullptr, h->q, 0.f, 0.f, 0.f,
                      DotOut{h->p, h->partials, h->st}, (const float*)nullptr, 0.f);
     } else

@@ -229,7 +229,7 @@ __device__ __forceinline__ double march_leaf(const LV& L, int leaf, int X0, bool
                 if constexpr (T::SCALED && DOTK == 0) rr = ld4(dot.r, leaf, (X0 + i) * 16 + q);
                 const double s = (double)res.x * rr.x + (double)res.y * rr.y + (double)res.z * rr.z +
                                  (double)res.w * rr.w;
-                if (on) sum += s;
+                if (on) sum = NP == 1 ? s : sum + s;
             }
         }
     };
@@ -319,9 +319,33 @@ __device__ __forceinline__ double march_leaf(const LV& L, int leaf, int X0, bool
     return sum;
 }
 
+// The block's part of a dot product into slot `slot` of `count`; the last block updates the PCG's scalars.
+template <int DOTK>
+__device__ __forceinline__ void march_dot(double sum, const DotOut& dot, int slot, int count) {
+    __shared__ double shd[MARCH_THREADS / 32];
+    const double part = block_sum128(sum, shd);
+    double tot = 0.0;
+    constexpr int TK = DOTK == 1 ? 2 : 0;
+    if (reduce_sum(part, dot.partials, &dot.st->ticket[TK], slot, count, tot) && threadIdx.x == 0) {
+        PcgState* st = dot.st;
+        if constexpr (DOTK == 1) {
+            const float sigma = (float)tot;
+            st->sigma = sigma;
+            st->alpha = __fdiv_rn(st->rho, sigma);
+            st->first = 0;
+        } else {
+            const float rho_new = (float)tot;
+            st->rho_new = rho_new;
+            st->beta = st->first ? 0.f : __fdiv_rn(rho_new, st->rho);
+            st->rho = rho_new;
+        }
+        st->ticket[TK] = 0;
+    }
+}
+
 // One pass over a level (march_leaf).  The dot products: rho and beta (PCG lines
 // 13-15, DOTK 0), or sigma and alpha (lines 6-7, DOTK 1); a partial per CTA, in
-// an order that depends on the level only.
+// an order that depends on the level only (NP 1: a CTA is a leaf, its threads those of the one-leaf kernels).
 template <int MODE, class LV, typename TOut, bool RESTRICT, int NP, int DOTK = 0>
 __global__ void __launch_bounds__(MARCH_THREADS, PipeLv<LV>::SCALED ? MARCH_MINB16 : MARCH_MINB)
     k_march(LV L, const typename PipeLv<LV>::E* x, const typename PipeLv<LV>::E* b, TOut* out, float w, float wsor,
@@ -333,28 +357,7 @@ __global__ void __launch_bounds__(MARCH_THREADS, PipeLv<LV>::SCALED ? MARCH_MINB
     const double sum = march_leaf<MODE, LV, TOut, RESTRICT, NP, DOTK>(L, leaf, X0, on, x, b, out, w, wsor, one_minus_wsor,
                                                                        dot, zscale, coarse_scale);
     if constexpr (!RESTRICT) {
-        if (dot.r) {
-            __shared__ double shd[MARCH_THREADS / 32];
-            const double part = block_sum128(sum, shd);
-            double tot = 0.0;
-            constexpr int TK = DOTK == 1 ? 2 : 0;
-            if (reduce_sum(part, dot.partials, &dot.st->ticket[TK], (int)blockIdx.x, (int)gridDim.x, tot) &&
-                threadIdx.x == 0) {
-                PcgState* st = dot.st;
-                if constexpr (DOTK == 1) {
-                    const float sigma = (float)tot;
-                    st->sigma = sigma;
-                    st->alpha = __fdiv_rn(st->rho, sigma);
-                    st->first = 0;
-                } else {
-                    const float rho_new = (float)tot;
-                    st->rho_new = rho_new;
-                    st->beta = st->first ? 0.f : __fdiv_rn(rho_new, st->rho);
-                    st->rho = rho_new;
-                }
-                st->ticket[TK] = 0;
-            }
-        }
+        if (dot.r) march_dot<DOTK>(sum, dot, (int)blockIdx.x, (int)gridDim.x);
     }
 }
 
