@@ -427,7 +427,7 @@ struct uaamg_poisson {
     cudaGraph_t graph = nullptr;
     int graph_key = -1;
     std::shared_ptr<struct SolveGraph> shared_graph;  // set when graph / graph_exec belong to the solve-graph cache
-    bool use_sweep2 = true;  // fused Jacobi sweep pairs (Enq::pair), fixed at creation
+    bool use_sweep2 = true;  // fused sweep pairs (Enq::pair), fixed at creation
     int64_t body_launches = 0, setup_launches = 0, finish_launches = 0;
     int64_t launches = 0;
     int64_t last_launches = 0;
@@ -1004,7 +1004,7 @@ static bool g_use_pdl = true;
 // Level sweeps with SrcPlain on levels of at least STAGED_MIN_LEAVES leaves run
 // the bulk-async staged kernels (UAAMG_STAGED=0 turns them off).
 static bool g_use_staged = true;
-static bool g_use_sweep2 = true;  // fused Jacobi sweep pairs (Enq::pair)
+static bool g_use_sweep2 = true;  // fused sweep pairs (Enq::pair)
 // Kernel shapes by level size (uaamg_set_tuning): the defaults below, or the
 // table an autotuner wrote.  Every choice gives the same results; only the
 // speed differs.  g_tune_gen is part of every graph's key, so a change rebuilds
@@ -1274,19 +1274,24 @@ struct Enq {
         count++;
     }
     bool split(int l) const { return g_use_staged && h->lv[l].L.nl >= SPLIT_MIN_LEAVES; }
-    // whether two consecutive Jacobi sweeps of level l run as one k_sweep2:
-    // latency-bound levels of about one wave at 2 CTAs per SM (from the staged
-    // size on); on larger levels the face-layer recomputation costs more than
-    // the launch it saves (measured: 776 and 784 leaves slower, 120-284 faster)
-    bool pair(int l) const {
-        const int nl = h->lv[l].L.nl;
-        return h->use_sweep2 && !split(l) && nl >= STAGED_MIN_LEAVES && nl <= 2 * g_sms;
+    // whether two consecutive Jacobi sweeps of level l, or the two colours of a
+    // Gauss-Seidel sweep, run as one k_sweep2: latency-bound levels of about one
+    // wave at 2 CTAs per SM; on larger levels the face-layer recomputation costs
+    // more than the launch it saves (Jacobi: 776 and 784 leaves slower, 120-284
+    // faster; red-black: 456 leaves slower, 5-284 faster).  Red-black solves, two
+    // launches a sweep / one: 64^3 (284, 40, 8 leaves) 770 / 660 us, 96^3 (776,
+    // 120, 19, 5) 1406 / 1166, 24^3 (19, 5) 457 / 397.
+    bool pair(int l) const { return h->use_sweep2 && !split(l) && h->lv[l].L.nl <= 2 * g_sms; }
+    template <int MA, int MB, class Src>
+    void sweep2_rb(int l, const Src& src, const float* b, float* out) {
+        const float ws = h->lv[l].w_sor;
+        sweep2<MA, MB>(l, src, b, out, ws, 1.0f - ws);
     }
-    template <class Src>
+    template <int MA = M_JACOBI, int MB = M_JACOBI, class Src>
     void sweep2(int l, const Src& src, const float* b, float* out, float wa, float wb) {
         LevelDev& D = h->lv[l];
-        if (prof) pb("L" + std::to_string(l) + " jacobi pair" + SrcName<Src>::get());
-        launch(k_sweep2<Src>, (unsigned)D.L.nl, SW2_THREADS, s, D.L, src, b, out, wa, wb);
+        if (prof) pb("L" + std::to_string(l) + " " + (MA == M_JACOBI ? "jacobi" : "red-black") + " pair" + SrcName<Src>::get());
+        launch(k_sweep2<MA, MB, Src>, (unsigned)D.L.nl, SW2_THREADS, s, D.L, src, b, out, wa, wb);
         pe();
         count++;
     }
@@ -1437,14 +1442,30 @@ static void enqueue_precond(Enq& E, int l, float* lhs, const float* rhs, bool sk
     auto wpre = [&](int i) { return sm == UAAMG_SMOOTHER_WEIGHTED_JACOBI ? 6.0f / 7.0f : sched_weight_precond(n, i); };
     float* cur = nullptr;
     if (sm == UAAMG_SMOOTHER_RED_BLACK_GAUSS_SEIDEL) {
-        int i0 = 0;
-        if (skip_first) {
-            E.sweep<M_BLACK>(l, SrcFirstRbgs{rhs, D.w_sor, 1}, rhs, lhs, 0.f);
-            i0 = 1;
-        }
-        for (int i = i0; i < n; ++i) {
-            E.sweep<M_RED>(l, SrcPlain{lhs}, rhs, lhs, 0.f);
+        const bool pair = E.pair(l);
+        if (pair && skip_first) {  // black, red | black, red | black
+            E.sweep2_rb<M_BLACK, M_RED>(l, SrcFirstRbgs{rhs, D.w_sor, 1}, rhs, D.tmp2);
+            E.sweep2_rb<M_BLACK, M_RED>(l, SrcPlain{D.tmp2}, rhs, lhs);
             E.sweep<M_BLACK>(l, SrcPlain{lhs}, rhs, lhs, 0.f);
+        } else if (pair) {
+            E.sweep2_rb<M_RED, M_BLACK>(l, SrcPlain{lhs}, rhs, D.tmp2);
+            E.sweep2_rb<M_RED, M_BLACK>(l, SrcPlain{D.tmp2}, rhs, T);
+            E.sweep2_rb<M_RED, M_BLACK>(l, SrcPlain{T}, rhs, lhs);
+        } else {
+            int i0 = 0;
+            if (skip_first) {
+                if (E.split(l)) {
+                    E.materialize(l, SrcFirstRbgs{rhs, D.w_sor, 1}, T);
+                    E.sweep<M_BLACK>(l, SrcPlain{T}, rhs, lhs, 0.f);
+                } else {
+                    E.sweep<M_BLACK>(l, SrcFirstRbgs{rhs, D.w_sor, 1}, rhs, lhs, 0.f);
+                }
+                i0 = 1;
+            }
+            for (int i = i0; i < n; ++i) {
+                E.sweep<M_RED>(l, SrcPlain{lhs}, rhs, lhs, 0.f);
+                E.sweep<M_BLACK>(l, SrcPlain{lhs}, rhs, lhs, 0.f);
+            }
         }
         cur = lhs;
         E.restrict_resid(l, cur, rhs);
@@ -1452,6 +1473,17 @@ static void enqueue_precond(Enq& E, int l, float* lhs, const float* rhs, bool sk
         if (l + 1 != h->nlev - 1) enqueue_precond(E, l + 1, P.lhs, P.rhs, false, DotOut{nullptr, nullptr, nullptr});
         // post: (black, red) x n; the first black pass adds the prolongation,
         // writes T; the last red pass writes back into lhs
+        if (pair) {
+            E.sweep2_rb<M_BLACK, M_RED>(l, SrcProlong{lhs, P.lhs, 1.0f}, rhs, D.tmp2);
+            E.sweep2_rb<M_BLACK, M_RED>(l, SrcPlain{D.tmp2}, rhs, T);
+            if (dot.r) {
+                E.sweep<M_BLACK>(l, SrcPlain{T}, rhs, T, 0.f);
+                E.sweep<M_RED>(l, SrcPlain{T}, rhs, lhs, 0.f, dot);
+            } else {
+                E.sweep2_rb<M_BLACK, M_RED>(l, SrcPlain{T}, rhs, lhs);
+            }
+            return;
+        }
         if (E.split(l)) {
             E.materialize(l, SrcProlong{lhs, P.lhs, 1.0f}, lhs);
             E.sweep<M_BLACK>(l, SrcPlain{lhs}, rhs, T, 0.f);

@@ -531,7 +531,8 @@ __global__ void __launch_bounds__(128) k_sweep(DLevel L, Src src, const float* b
 }
 
 // ---------------------------------------------------------------------------
-// Two Jacobi sweeps in one launch: out = J_wb(J_wa(src)).  The second sweep at a
+// Two sweeps in one launch: Jacobi, out = J_wb(J_wa(src)), or the two colours of
+// Gauss-Seidel, MA then MB (wa = w_sor, wb = 1 - w_sor).  The second sweep at a
 // voxel reads the first sweep's result at its six neighbours, so a CTA computes
 // the first sweep for its leaf and for the face layers of its six neighbours
 // (the values the neighbouring CTAs compute too, from the same inputs with the
@@ -545,9 +546,10 @@ __global__ void __launch_bounds__(128) k_sweep(DLevel L, Src src, const float* b
 // thread is not their z-line's other half).
 #define SW2_THREADS 320
 __device__ __forceinline__ int sw2_idx(int X, int Y, int Z) { return ((X + 1) * 10 + (Y + 1)) * 10 + (Z + 1); }
-template <class Src>
+template <int MA, int MB, class Src>
 __global__ void __launch_bounds__(SW2_THREADS, 2) k_sweep2(DLevel L, Src src, const float* b, float* out, float wa,
                                                            float wb) {
+    constexpr bool GS = MA != M_JACOBI;
     __shared__ float cube[1000];
     const int t = threadIdx.x;
     const int leaf = blockIdx.x;
@@ -579,13 +581,14 @@ __global__ void __launch_bounds__(SW2_THREADS, 2) k_sweep2(DLevel L, Src src, co
         cZ0 = zf ? 8 : -4;
     }
     SStatic S;
-    if (gl >= 0) sweep_static<M_JACOBI>(L, gl, gt, S);
+    if (gl >= 0) sweep_static<MA>(L, gl, gt, S);
     griddep_wait();
     griddep_launch();
     float4 T = f4zero(), xc;
     unsigned m = 0;
-    if (t < 128) T = sweep_value_s<M_JACOBI, Src, true>(L, leaf, t, src, b, wa, 0.f, 1.f, S, xc, m);
-    else if (gl >= 0) T = sweep_value_s<M_JACOBI, Src, false>(L, gl, gt, src, b, wa, 0.f, 1.f, S, xc, m);
+    const float w0 = GS ? 0.f : wa, ws = GS ? wa : 0.f, wr = GS ? wb : 1.f;
+    if (t < 128) T = sweep_value_s<MA, Src, true>(L, leaf, t, src, b, w0, ws, wr, S, xc, m);
+    else if (gl >= 0) T = sweep_value_s<MA, Src, false>(L, gl, gt, src, b, w0, ws, wr, S, xc, m);
     if (zlane < 0) {
         const int base = sw2_idx(cX, cY, cZ0);
         cube[base] = T.x;
@@ -623,9 +626,17 @@ __global__ void __launch_bounds__(SW2_THREADS, 2) k_sweep2(DLevel L, Src src, co
     float4 res;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        float r = __fsub_rn(f4get(bb, j), __fmaf_rn(f4get(T, j), f4get(S.dg, j), f4get(off, j)));
-        r = __fmul_rn(r, f4get(S.iv, j));
-        f4set(res, j, __fmaf_rn(wb, r, f4get(T, j)));
+        if constexpr (GS) {
+            float r = __fsub_rn(f4get(bb, j), f4get(off, j));
+            r = __fmul_rn(r, f4get(S.iv, j));
+            r = __fmul_rn(r, wa);
+            const float v = __fmaf_rn(f4get(T, j), wb, r);
+            f4set(res, j, ((X + Y + j) & 1) == (MB == M_RED ? 0 : 1) ? v : f4get(T, j));
+        } else {
+            float r = __fsub_rn(f4get(bb, j), __fmaf_rn(f4get(T, j), f4get(S.dg, j), f4get(off, j)));
+            r = __fmul_rn(r, f4get(S.iv, j));
+            f4set(res, j, __fmaf_rn(wb, r, f4get(T, j)));
+        }
     }
     if (!(m & 1)) res.x = 0.f;
     if (!(m & 2)) res.y = 0.f;
