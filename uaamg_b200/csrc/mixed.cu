@@ -228,10 +228,10 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     const float* ns = nullptr;
     if (l == last) {
         if (M->nc > 0) {
-            const unsigned rows = (unsigned)((M->nc + 7) / 8);
+            const unsigned ctas = (unsigned)((M->nc + CGEMV_CTA_ROWS - 1) / CGEMV_CTA_ROWS);
             cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(rows);
-            cfg.blockDim = dim3(256);
+            cfg.gridDim = dim3(ctas);
+            cfg.blockDim = dim3(CGEMV_THREADS);
             cfg.dynamicSmemBytes = (size_t)M->nc * sizeof(double);
             cfg.stream = E.s;
             cudaLaunchAttribute at[1];

@@ -752,23 +752,52 @@ __global__ void __launch_bounds__(256) k_gj_update(double* A, int n, int k, cons
         A[idx] = a - fcol[i] * rrow[j];
     }
 }
-// out(slot i) = sum_j Ainv[i][j] rhs(slot j): one warp per row, FP64
+// out(slot i) = sum_j Ainv[i][j] rhs(slot j), FP64: CGEMV_ROWS rows per warp,
+// CGEMV_AHEAD values of each loaded before they are added (lane after lane, in
+// order of j).  The matrix's bytes bound it (3,884 DOF: 121 MB, 18 us); the first
+// values load while the previous kernel still runs.  One row per warp and a
+// block's gather of the rhs for eight rows took 45 us by events around the launch, this 30 (four rows of
+// four values 40, one row of sixteen 30), and a 320^3 FP16 solve 9.2 ms, now 7.5.
+constexpr int CGEMV_ROWS = 2, CGEMV_AHEAD = 8, CGEMV_THREADS = 256;
+constexpr int CGEMV_CTA_ROWS = CGEMV_THREADS / 32 * CGEMV_ROWS;
 template <typename T>
-__global__ void __launch_bounds__(256) k_cgemv(int n, const double* Ainv, const int* slot, const T* rhs, T* out,
-                                               float rhs_scale) {
+__global__ void __launch_bounds__(CGEMV_THREADS) k_cgemv(int n, const double* Ainv, const int* slot, const T* rhs, T* out,
+                                                         float rhs_scale) {
+    extern __shared__ double bs[];
+    const int lane = threadIdx.x & 31, row0 = blockIdx.x * CGEMV_CTA_ROWS + (threadIdx.x >> 5) * CGEMV_ROWS;
+    const double* a[CGEMV_ROWS];
+    double v[CGEMV_ROWS][CGEMV_AHEAD];
+    auto load = [&](int j) {
+#pragma unroll
+        for (int r = 0; r < CGEMV_ROWS; ++r)
+#pragma unroll
+            for (int u = 0; u < CGEMV_AHEAD; ++u) v[r][u] = j + 32 * u < n ? __ldcs(a[r] + j + 32 * u) : 0.0;
+    };
+#pragma unroll
+    for (int r = 0; r < CGEMV_ROWS; ++r) a[r] = Ainv + (long long)min(row0 + r, n - 1) * n;
+    load(lane);
     griddep_wait();
     griddep_launch();
-    extern __shared__ double bs[];
-    for (int j = threadIdx.x; j < n; j += blockDim.x) bs[j] = (double)ldh1(rhs, slot[j]) * (double)rhs_scale;
+#pragma unroll 4
+    for (int j = threadIdx.x; j < n; j += CGEMV_THREADS) bs[j] = (double)ldh1(rhs, slot[j]) * (double)rhs_scale;
     __syncthreads();
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const double* a = Ainv + (long long)row * n;
-    double s = 0.0;
-    for (int j = lane; j < n; j += 32) s += a[j] * bs[j];
+    double s[CGEMV_ROWS] = {};
+    for (int j = lane; j < n; j += 32 * CGEMV_AHEAD) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(FULLMASK, s, o);
-    if (lane == 0) out[slot[row]] = H16<T>::from1((float)s);
+        for (int u = 0; u < CGEMV_AHEAD; ++u) {
+            if (j + 32 * u >= n) break;
+            const double x = bs[j + 32 * u];
+#pragma unroll
+            for (int r = 0; r < CGEMV_ROWS; ++r) s[r] += v[r][u] * x;
+        }
+        if (j + 32 * CGEMV_AHEAD < n) load(j + 32 * CGEMV_AHEAD);
+    }
+#pragma unroll
+    for (int r = 0; r < CGEMV_ROWS; ++r) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_down_sync(FULLMASK, s[r], o);
+        if (lane == 0 && row0 + r < n) out[slot[row0 + r]] = H16<T>::from1((float)s[r]);
+    }
 }
 
 // r = b - A x every `every` iterations of the outer CG (true-residual
