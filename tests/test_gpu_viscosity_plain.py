@@ -44,3 +44,22 @@ def test_plain_leaves_equal(gpu, monkeypatch, n, fill):
     assert np.array_equal(z0, z1)
     assert a == b and a[0] == 0
     assert np.array_equal(x0, x1)
+
+
+def test_precondition_zero_outside_dof(gpu):
+    """Level 0 is the bottom level at 24^3: the cycle writes its DOF only, and the
+    result is zero elsewhere whatever the memory held before."""
+    import gc
+    from uaamg_b200.viscosity import L_with_level, simd_viscosity3d
+    sc = scenes.plain_viscosity_scene(n=24, seed=2)
+    for _ in range(3):
+        lv = L_with_level.create_viscosity_matrix(sc.viscosity, sc.liquid_phi, sc.solid_phi, sc.dt, sc.rho, sc.dx)
+        assert lv.num_levels() == 2
+        rhs = lv.build_rhs(sc.u, sc.v, sc.w, sc.solid_velocity)
+        s = simd_viscosity3d(lv)
+        z = s.precondition(np.ones_like(rhs))
+        assert not z[np.asarray(lv.dof_index(0)).reshape(z.shape) < 0].any()
+        x = lv.gather_velocity(sc.u, sc.v, sc.w)
+        s.pcg_solve(x, 1e-6, rhs)
+        del s, lv
+        gc.collect()

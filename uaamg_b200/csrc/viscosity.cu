@@ -1580,6 +1580,7 @@ int uaamg_viscosity_precondition(uaamg_viscosity* h, const float* r, float* z) {
     float* rr = sc.get(vb);
     float* zz = sc.get(vb);
     CK(cudaMemcpyAsync(rr, r, vb, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemsetAsync(zz, 0, vb, h->stream));  // a bottom cycle or coarsest solve on level 0 writes the DOF only
     launch2(k_vmask, dim3((unsigned)h->lv[0].L.nl, 3), 128, h->stream, h->lv[0].L, rr);
     VEnq E{h, h->stream};
     enqueue_mucycle(E, 0, zz, rr, true);
