@@ -492,10 +492,11 @@ static void build_vbottom(uaamg_viscosity* h) {
     for (;; ++NC) {
         if (NC > hi) return;
         int cap = 0;
-        for (int g = 0; g < 6; ++g) cap += (R.gs[g + 1] - R.gs[g] + NC - 1) / NC;
+        for (int g = 0; g < 6; ++g) cap += vb_part(R.gs[g + 1] - R.gs[g], NC, 0).cnt;
         smem = (rows ? vbot_layout<4>(R.n, nc, cap) : vbot_layout<0>(R.n, nc, cap)).total;
         if (smem <= (size_t)max_dynamic) break;
     }
+    for (int g = 0; g <= VB_GROUPS; ++g) R.val[g] = vb_values(R.gs, NC, g);
     if (!cluster_fits(vbottom_kernel(rows), NC + (rows ? 1 : 0), VB_THREADS, smem, max_dynamic)) return;
     const size_t n = (size_t)R.n;
     int* dbase = vupload(h, base.data(), base.size());

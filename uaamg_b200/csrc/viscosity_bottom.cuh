@@ -18,14 +18,21 @@
 // mbarrier.  So one one-way trip through the cluster separates two passes; no
 // barrier of the cluster and no fence is on that path.
 //
-// Measured (events around the launch): 128^3, two visits with their CG 66 us,
-// 54 launches of 2.2 us in a graph before; 44^3 (15,496 DOF over 2,017) 98 us
+// Measured (events around the launch): 128^3, two visits with their CG 68 us,
+// 54 launches of 2.2 us in a graph before; 44^3 (15,496 DOF over 2,017) 99 us
 // against 57 launches, whole solve 7.4 -> 4.8 ms as a graph.
 //
-// Why this is safe without one: a CTA sends pass p + 1 only when all of pass p
-// has arrived, and a row's value is sent after its gathers, so when a value of
-// pass p + 1 arrives anywhere every gather of pass p is done.  Two mbarriers
-// alternate, because a sender may be one pass ahead of a receiver, never two.
+// Why this is safe without one: a warp sends pass p + 1 only when all of pass p
+// has arrived, and a row's value is sent after its gathers; so when a value of
+// pass p + 1 arrives anywhere, every gather of pass p is done.  Every CTA sends
+// in every pass, one word that nobody reads where it has no row of the group
+// (viscosity_split.h), so all of a pass arrives only when every CTA is in it.
+// Two mbarriers, a parity bit each, alternate: a warp has to see pass p's phase
+// before pass p + 2's ends.  The warps of a CTA that have rows (the others take
+// no part) meet at a named barrier after each pass, so none of them sends p + 1
+// while another still waits for p.  (That and the words: 65.6 -> 68.2 us a
+// launch at 128^3, 98.5 -> 98.6 at 44^3.  A barrier after every second pass
+// would do, but 68.6 and 100.7: the warps drift apart.)
 //
 // The coarsest CG runs in a CTA of its own while its rows fit that CTA's
 // registers (up to 1024 DOF, k_vcoarsest_cg's form), above that over eight
@@ -35,6 +42,7 @@
 #include <cooperative_groups.h>
 
 #include "viscosity_kernels.cuh"
+#include "viscosity_split.h"
 
 namespace uaamg {
 
@@ -46,6 +54,7 @@ namespace uaamg {
 struct VBotRows {        // level lb by DOF, rows sorted by group channel * 2 + colour
     int n, nc;           // rows; coarsest DOFs
     int gs[7];           // first row of each group
+    int val[7];          // values a row CTA receives in a pass over the group (vb_values; [6]: over all rows)
     const float* coef;   // [14][n]: neg +x, -x, +y, -y, +z, -z; T of channel d2: 00 01 10 11; T of channel d1: the same
     const unsigned* idx; // [7][n] rows of the values they multiply, two 16-bit ones per word; n = no DOF
     const float* iv;     // [n] 1/diag
@@ -454,7 +463,8 @@ template <int ROWS>
 __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
     extern __shared__ __align__(16) unsigned char vsm[];
     __shared__ uint64_t bars[4];                  // x (two that alternate), residuals, coarse solution
-    __shared__ int g_row[6], g_cnt[6], g_loc[7];  // this CTA's rows of each group: first, count, local position
+    __shared__ int g_row[6], g_cnt[7], g_loc[6];  // this CTA's rows of each group: first, count, local position
+    __shared__ float g_word;                      // where the words of CTAs without rows arrive
     constexpr unsigned R0 = ROWS ? 1u : 0u;       // first row CTA
     const unsigned rank = cooperative_groups::this_cluster().block_rank();
     const int t = threadIdx.x, n = A.R.n, nc = A.R.nc, NC = A.NC;
@@ -507,14 +517,13 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
     if (t == 0) {
         int at = 0;
         for (int g = 0; g < 6; ++g) {
-            const int size = A.R.gs[g + 1] - A.R.gs[g], s = (size + NC - 1) / NC;
-            const int lo = min(j * s, size), hi = min(lo + s, size);
-            g_row[g] = A.R.gs[g] + lo;
-            g_cnt[g] = hi - lo;
+            const VbPart part = vb_part(A.R.gs[g + 1] - A.R.gs[g], NC, j);
+            g_row[g] = A.R.gs[g] + part.lo;
+            g_cnt[g] = part.cnt;
             g_loc[g] = at;
-            at += hi - lo;
+            at += part.cnt;
         }
-        g_loc[6] = at;
+        g_cnt[6] = at;
     }
     float* x = reinterpret_cast<float*>(vsm + o.x);
     float* xc = reinterpret_cast<float*>(vsm + o.xc);
@@ -561,6 +570,8 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
     __syncthreads();
     vb_cluster_sync();  // every CTA has started, its mbarriers and its copy are set up
 
+    const int nthr = vb_threads(g_cnt, VB_THREADS);
+    const bool active = t < nthr;  // (uniform in a warp)
     const VbSm s{scoef, siv, sb, sidx, cap};
     const unsigned xb = smem_u32(x);
     int pass = 0;  // exchanges of x so far
@@ -568,55 +579,63 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
     auto fetch = [&](int g) {
         if (t < g_cnt[g]) vb_row(s, g_loc[g] + t, nx);
     };
-    auto arm = [&](int rows) {
-        if (t == 0) vb_arm(bx + 8u * (pass & 1), 4u * (unsigned)rows);
+    auto arm = [&](int g) {  // a pass over group g (6: all rows) begins
+        if (t == 0) vb_arm(bx + 8u * (pass & 1), 4u * (unsigned)A.R.val[g]);
+    };
+    auto put = [&](unsigned a, float v) {
+        for (int q = 0; q < NC; ++q) vb_send(a, bx + 8u * (pass & 1), R0 + (unsigned)q, v);
+    };
+    auto send = [&](int row, float v) { put(xb + 4u * (unsigned)row, v); };
+    auto sent = [&](int cnt) {  // the rows' values are sent; a CTA without rows sends its word
+        if (cnt == 0 && t == 0) put(smem_u32(&g_word), 0.f);
     };
     auto wait = [&]() {
         vb_wait(bx + 8u * (pass & 1), (pass >> 1) & 1, A.error, dead);
         ++pass;
-    };
-    auto send = [&](int row, float v) {
-        for (int q = 0; q < NC; ++q) vb_send(xb + 4u * (unsigned)row, bx + 8u * (pass & 1), R0 + (unsigned)q, v);
+        asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
     };
     // one Gauss-Seidel pass over group g; next: the group whose first row to fetch meanwhile (-1: none)
     auto gauss_seidel = [&](int g, int next) {
-        arm(A.R.gs[g + 1] - A.R.gs[g]);
+        arm(g);
         const int cnt = g_cnt[g], row0 = g_row[g], loc = g_loc[g];
         for (int i = t; i < cnt; i += VB_THREADS) {
             if (i != t) vb_row(s, loc + i, nx);
             send(row0 + i, vgs_update(nx.b, vb_off(nx, x), nx.iv, 1.0f, 0.0f, x[row0 + i]));
         }
+        sent(cnt);
         if (next >= 0) fetch(next);
         wait();
     };
 #pragma unroll 1
     for (int visit = 0; visit < A.visits; ++visit) {
-        fetch(0);
-#pragma unroll 1
-        for (int q = 0; q < 12; ++q) gauss_seidel(q % 6, q < 11 ? (q + 1) % 6 : -1);  // x, y, z: red, black
-        // residuals to where they are restricted
         if constexpr (ROWS == 0) {
             if (cg8 && t == 0) vb_arm(bres, 4u * (unsigned)rexp);
         }
+        if (active) {
+            fetch(0);
 #pragma unroll 1
-        for (int g = 0; g < 6; ++g) {
-            const int cnt = g_cnt[g], row0 = g_row[g], loc = g_loc[g];
-            for (int i = t; i < cnt; i += VB_THREADS) {
-                VbRow w;
-                vb_row(s, loc + i, w);
-                const float res = __fsub_rn(w.b, __fmaf_rn(x[row0 + i], sdg[loc + i], vb_off(w, x)));
-                const int cd = scd[loc + i];
-                if constexpr (ROWS > 0) {
-                    vb_send(smem_u32(vsm) + 4u * (unsigned)cd, bres, 0u, res);
-                } else {
-                    const int cr = cd >> 3, pos = (((cr >> 8) << 5) | (cr & 31)) * 8 + (cd & 7);
-                    vb_send(smem_u32(rbuf) + 4u * (unsigned)pos, bres, (unsigned)((cr & 255) >> 5), res);
+            for (int q = 0; q < 12; ++q) gauss_seidel(q % 6, q < 11 ? (q + 1) % 6 : -1);  // x, y, z: red, black
+            // residuals to where they are restricted
+#pragma unroll 1
+            for (int g = 0; g < 6; ++g) {
+                const int cnt = g_cnt[g], row0 = g_row[g], loc = g_loc[g];
+                for (int i = t; i < cnt; i += VB_THREADS) {
+                    VbRow w;
+                    vb_row(s, loc + i, w);
+                    const float res = __fsub_rn(w.b, __fmaf_rn(x[row0 + i], sdg[loc + i], vb_off(w, x)));
+                    const int cd = scd[loc + i];
+                    if constexpr (ROWS > 0) {
+                        vb_send(smem_u32(vsm) + 4u * (unsigned)cd, bres, 0u, res);
+                    } else {
+                        const int cr = cd >> 3, pos = (((cr >> 8) << 5) | (cr & 31)) * 8 + (cd & 7);
+                        vb_send(smem_u32(rbuf) + 4u * (unsigned)pos, bres, (unsigned)((cr & 255) >> 5), res);
+                    }
                 }
             }
+            if (t == 0) vb_arm(bxc, 4u * (unsigned)nc);
         }
-        if (t == 0) vb_arm(bxc, 4u * (unsigned)nc);
         if constexpr (ROWS == 0) {
-            if (cg8) {
+            if (cg8) {  // the whole block
                 vb_wait(bres, visit & 1, A.error, dead);
                 const int w = t >> 5, l = t & 31;
                 float r[2], cx[2];
@@ -633,13 +652,15 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
                             vb_send(smem_u32(xc) + 4u * (unsigned)M.row[q], bxc, (unsigned)k, cx[q]);
             }
         }
+        if (!active) continue;
         vb_wait(bxc, visit & 1, A.error, dead);
         // prolongation: x += x_c of the coarse voxel
-        arm(n);
+        arm(6);
 #pragma unroll 1
         for (int g = 0; g < 6; ++g)
             for (int i = t; i < g_cnt[g]; i += VB_THREADS)
                 send(g_row[g] + i, __fadd_rn(x[g_row[g] + i], xc[scd[g_loc[g] + i] >> 3]));
+        sent(g_cnt[6]);
         fetch(5);
         wait();
 #pragma unroll 1
