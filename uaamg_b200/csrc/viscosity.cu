@@ -312,6 +312,7 @@ struct uaamg_viscosity {
     VBotRows bot{};
     int bot_NC = 0, bot_rows = 0;
     size_t bot_smem = 0;
+    unsigned long long wait_ns = 2000000000;  // how long the CTAs of a bottom cycle or coarsest solve wait for one another
     float *x = nullptr, *b = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;
     double* partials = nullptr;
     PcgState* st = nullptr;
@@ -848,12 +849,13 @@ struct VEnq {
         pe();
         count++;
     }
+    VbLimit limit() const { return VbLimit{h->wait_ns, &h->st->error}; }
     void coarsest(const float* rhs, float* out) {
         if (h->C.n == 0) return;
         if (prof) pb("coarsest cg");
         if (h->C.n <= 2 * VCG_THREADS) launch2(k_vcoarsest_cg<2>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
         else if (vbottom_cg_rows(h->C.n)) launch2(k_vcoarsest_cg<4>, dim3(1), VCG_THREADS, s, h->C, rhs, out);
-        else launch_cluster(k_vcoarsest_cg8, VB_CG8, VB_THREADS, vcg8_smem_bytes(h->C.n), s, h->C, rhs, out, &h->st->error);
+        else launch_cluster(k_vcoarsest_cg8, VB_CG8, VB_THREADS, vcg8_smem_bytes(h->C.n), s, h->C, rhs, out, limit());
         pe();
         count++;
     }
@@ -868,7 +870,7 @@ struct VEnq {
         A.visits = h->nlev == 2 ? 1 : 2;
         A.rhs = rhs;
         A.lhs = lhs;
-        A.error = &h->st->error;
+        A.lim = limit();
         if (prof) pb("L" + std::to_string(h->nlev - 2) + " bottom (visits + coarsest)");
         launch_cluster(vbottom_kernel(h->bot_rows), h->bot_NC + (h->bot_rows ? 1 : 0), VB_THREADS, h->bot_smem, s, A);
         pe();
@@ -1119,7 +1121,7 @@ static int vrun_pcg(uaamg_viscosity* h, std::vector<ProfRec>* prof = nullptr) {
     h->launches += launches;
     const PcgState& s = *h->st_host;
     if (s.error) {
-        set_error("a kernel's bounded wait for its bulk copies timed out");
+        set_error("the CTAs of a bottom cycle or coarsest solve waited too long for one another");
         throw UaamgError{UAAMG_ERR_CUDA};
     }
     h->iterations = s.iterations_taken;
@@ -1248,6 +1250,7 @@ int uaamg_viscosity_create_on_stream(const uaamg_leaf_grid* viscosity, const uaa
         h->seq_min_leaves = 2 * g_sms + 1;
         if (const char* e = getenv("UAAMG_VISC_FUSED_RB_LEAVES")) h->rb_fused_max_leaves = atoi(e);
         if (const char* e = getenv("UAAMG_VISC_SEQ_LEAVES")) h->seq_min_leaves = atoi(e);
+        if (const char* e = getenv("UAAMG_VISC_WAIT_US")) h->wait_ns = 1000ull * std::min(std::max(atol(e), 0L), 10000000L);
         if (const char* e = getenv("UAAMG_VISC_PLAIN_LEAVES")) h->plain_min_leaves = atoi(e);
         build_viscosity(h, viscosity, liquid_sdf, solid_sdf, dt, rho, dx);
     } catch (const UaamgError& e) {

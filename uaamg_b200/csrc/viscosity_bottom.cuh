@@ -63,6 +63,10 @@ struct VBotRows {        // level lb by DOF, rows sorted by group channel * 2 + 
     const uint16_t* cdst;  // [n] coarse DOF * 8 + octant in it
     const int* rcount;   // [8] rows whose coarse DOF each CTA of the distributed CG holds
 };
+struct VbLimit {            // of the waits of a cluster's CTAs for one another
+    unsigned long long ns;  // 0: every wait gives up at once
+    int* error;
+};
 struct VBotArgs {
     VBotRows R;
     DCoarsestV C;
@@ -70,7 +74,7 @@ struct VBotArgs {
     int visits;        // 2, or 1 when level lb is the top
     const float* rhs;  // level lb
     float* lhs;
-    int* error;
+    VbLimit lim;
 };
 
 // ---- building the rows -----------------------------------------------------
@@ -180,19 +184,35 @@ __device__ __forceinline__ bool vb_try_wait(unsigned bar, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-// Waits for a phase; gives up after 2^20 polls (each blocks briefly), then sets the error and waits no more.
-__device__ __forceinline__ void vb_wait(unsigned bar, unsigned parity, int* error, bool& dead) {
+__device__ __forceinline__ void vb_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned long long vb_now() {  // ns
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// Waits for a phase, within the limit (each poll blocks briefly).  A wait that
+// gives up sets the kernel's error word and `dead` in the thread, which from
+// then on neither waits, arms nor sends; nor do the launches after it, until
+// the word is cleared for the next solve.
+__device__ __forceinline__ void vb_wait(unsigned bar, unsigned parity, const VbLimit& lim, bool& dead) {
     if (dead) return;
-    for (int i = 0; i < (1 << 20); ++i)
+    if (lim.ns && vb_try_wait(bar, parity)) return;
+    for (const unsigned long long t0 = vb_now(); vb_now() - t0 < lim.ns;)
         if (vb_try_wait(bar, parity)) return;
     dead = true;
-    *error = 1;
+    *lim.error = 1;
+}
+// The last thing a CTA does: nobody sends into a CTA that has left.  After a
+// wait that gave up, values may still be under way to it when all have met.
+__device__ __forceinline__ void vb_leave(bool dead) {
+    __syncthreads();
+    vb_cluster_sync();
+    if (dead) __nanosleep(100000);
 }
 __device__ __forceinline__ void vb_arm(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void vb_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ---- the coarsest CG over eight CTAs ----------------------------------------
@@ -255,7 +275,7 @@ __device__ __forceinline__ void vcg8_init(const VCg8Smem& S) {
 }
 // this CTA's sums of ca * fb over its lanes' chains (and, second, of ca * cb): to every CTA
 __device__ __forceinline__ void vcg8_sum(const VCg8Smem& S, int kmax, int j, bool squares, bool products, float* dst,
-                                         unsigned bar, unsigned rank0) {
+                                         unsigned bar, unsigned rank0, bool dead) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int nsum = (int)squares + (int)products;
     if (w >= nsum) return;
@@ -267,12 +287,14 @@ __device__ __forceinline__ void vcg8_sum(const VCg8Smem& S, int kmax, int j, boo
     }
     acc = cg_warp_partial(acc);
     acc = __shfl_sync(FULLMASK, acc, 0);
-    if (l < VB_CG8) vb_send(smem_u32(dst + 8 * w + j), bar, rank0 + (unsigned)l, acc);
+    if (l < VB_CG8 && !dead) vb_send(smem_u32(dst + 8 * w + j), bar, rank0 + (unsigned)l, acc);
 }
 // x of this thread's rows for the rhs r (0 in rows it does not have); every thread of the eight CTAs.
-// ph: phases of the three mbarriers used so far (they advance together with the solves).
+// ph: phases of the three mbarriers used so far (they advance together with the solves).  Once a wait of one of its
+// threads gives up, a CTA's threads leave together (stop): the barriers inside are the whole block's.
 __device__ __forceinline__ void vcg8_solve(const DCoarsestV& C, const VCg8Rows& M, const VCg8Smem& S, int j, unsigned rank0,
-                                           float (&r)[2], float (&x)[2], unsigned (&ph)[3], int* error, bool& dead) {
+                                           float (&r)[2], float (&x)[2], unsigned (&ph)[3], const VbLimit& lim,
+                                           bool& dead) {
     const int t = threadIdx.x, w = t >> 5, l = t & 31;
     const int kmax = vcg8_kmax(C.n);
     const unsigned bp = smem_u32(&S.bar[0]), b1 = smem_u32(&S.bar[1]), b2 = smem_u32(&S.bar[2]);
@@ -287,18 +309,23 @@ __device__ __forceinline__ void vcg8_solve(const DCoarsestV& C, const VCg8Rows& 
         __syncthreads();
     };
     auto wait = [&](unsigned bar, int i) {
-        vb_wait(bar, ph[i] & 1u, error, dead);
+        vb_wait(bar, ph[i] & 1u, lim, dead);
         ph[i]++;
+    };
+    auto stop = [&]() {
+        dead = __syncthreads_or(dead) != 0;
+        return dead;
     };
     float p[2] = {0.f, 0.f}, z[2];
     x[0] = x[1] = 0.f;
     // r.r, then r.z with z = invd r
-    if (t == 0) vb_arm(b2, 64);
+    if (t == 0 && !dead) vb_arm(b2, 64);
 #pragma unroll
     for (int q = 0; q < 2; ++q) z[q] = __fmul_rn(M.iv[q], r[q]);
     factors(r, z);
-    vcg8_sum(S, kmax, j, true, true, S.s2, b2, rank0);
+    vcg8_sum(S, kmax, j, true, true, S.s2, b2, rank0, dead);
     wait(b2, 2);
+    if (stop()) return;
     const float rhsNorm2 = cg_tree_sum<8>(S.s2);
     float absNew = cg_tree_sum<8>(S.s2 + 8);
     const float threshold = fmaxf(__fmul_rn(__fmul_rn(FLT_EPSILON, FLT_EPSILON), rhsNorm2), FLT_MIN);
@@ -306,14 +333,14 @@ __device__ __forceinline__ void vcg8_solve(const DCoarsestV& C, const VCg8Rows& 
     p[0] = z[0];
     p[1] = z[1];
     for (int it = 0; it < 10; ++it) {
-        if (t == 0) {
+        if (t == 0 && !dead) {
             vb_arm(bp, 4u * (unsigned)C.n);
             vb_arm(b1, 32);
             vb_arm(b2, 64);
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q)
-            if (M.row[q] >= 0)
+            if (M.row[q] >= 0 && !dead)
 #pragma unroll
                 for (unsigned k = 0; k < VB_CG8; ++k) vb_send(pb + 4u * (unsigned)M.row[q], bp, rank0 + k, p[q]);
         wait(bp, 0);
@@ -329,7 +356,7 @@ __device__ __forceinline__ void vcg8_solve(const DCoarsestV& C, const VCg8Rows& 
             tq[q] = s;
         }
         factors(p, tq);
-        vcg8_sum(S, kmax, j, false, true, S.s1, b1, rank0);
+        vcg8_sum(S, kmax, j, false, true, S.s1, b1, rank0, dead);
         wait(b1, 1);
         const float alpha = __fdiv_rn(absNew, cg_tree_sum<8>(S.s1));
 #pragma unroll
@@ -339,8 +366,9 @@ __device__ __forceinline__ void vcg8_solve(const DCoarsestV& C, const VCg8Rows& 
             z[q] = __fmul_rn(M.iv[q], r[q]);
         }
         factors(r, z);
-        vcg8_sum(S, kmax, j, true, true, S.s2, b2, rank0);
+        vcg8_sum(S, kmax, j, true, true, S.s2, b2, rank0, dead);
         wait(b2, 2);
+        if (stop()) return;
         const float rr = cg_tree_sum<8>(S.s2);
         if (rr < threshold) break;
         const float absOld = absNew;
@@ -352,7 +380,7 @@ __device__ __forceinline__ void vcg8_solve(const DCoarsestV& C, const VCg8Rows& 
 }
 
 // the coarsest solve alone, for hierarchies whose level lb does not fit k_vbottom: one cluster of VB_CG8 CTAs
-__global__ void __launch_bounds__(VB_THREADS, 1) k_vcoarsest_cg8(DCoarsestV C, const float* rhs, float* out, int* error) {
+__global__ void __launch_bounds__(VB_THREADS, 1) k_vcoarsest_cg8(DCoarsestV C, const float* rhs, float* out, VbLimit lim) {
     extern __shared__ __align__(16) unsigned char cg8_mem[];
     const VCg8Smem S = vcg8_smem(cg8_mem, C.n);
     const int j = (int)cooperative_groups::this_cluster().block_rank();
@@ -370,13 +398,12 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vcoarsest_cg8(DCoarsestV C, c
 #pragma unroll
     for (int q = 0; q < 2; ++q) r[q] = sl[q] >= 0 ? rhs[sl[q]] : 0.f;
     unsigned ph[3] = {0, 0, 0};
-    bool dead = false;
-    vcg8_solve(C, M, S, j, 0, r, x, ph, error, dead);
+    bool dead = __ldcg(lim.error) != 0;
+    vcg8_solve(C, M, S, j, 0, r, x, ph, lim, dead);
 #pragma unroll
     for (int q = 0; q < 2; ++q)
         if (sl[q] >= 0) out[sl[q]] = x[q];
-    __syncthreads();
-    vb_cluster_sync();  // nobody sends into a CTA that has left
+    vb_leave(dead);
 }
 
 // ---- both visits ------------------------------------------------------------
@@ -488,11 +515,12 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
             vb_cluster_sync();
             griddep_wait();
             griddep_launch();
+            dead = __ldcg(A.lim.error) != 0;
             const unsigned xcb = smem_u32(vsm + o.xc);
 #pragma unroll 1
             for (int visit = 0; visit < A.visits; ++visit) {
-                if (t == 0) vb_arm(bres, 4u * (unsigned)n);
-                vb_wait(bres, visit & 1, A.error, dead);
+                if (t == 0 && !dead) vb_arm(bres, 4u * (unsigned)n);
+                vb_wait(bres, visit & 1, A.lim, dead);
                 float r[ROWS], x[ROWS];
 #pragma unroll
                 for (int k = 0; k < ROWS; ++k) {
@@ -503,12 +531,11 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
 #pragma unroll
                 for (int k = 0; k < ROWS; ++k) {
                     const int i = t + k * VCG_THREADS;
-                    if (i < nc)
+                    if (i < nc && !dead)
                         for (int q = 0; q < NC; ++q) vb_send(xcb + 4u * (unsigned)i, bxc, R0 + (unsigned)q, x[k]);
                 }
             }
-            __syncthreads();
-            vb_cluster_sync();
+            vb_leave(dead);
             return;
         }
     }
@@ -565,6 +592,7 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
     }
     griddep_wait();
     griddep_launch();
+    dead = __ldcg(A.lim.error) != 0;
     for (int g = 0; g < 6; ++g)
         for (int i = t; i < g_cnt[g]; i += VB_THREADS) sb[g_loc[g] + i] = A.rhs[A.R.slot[g_row[g] + i]];
     __syncthreads();
@@ -580,9 +608,10 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
         if (t < g_cnt[g]) vb_row(s, g_loc[g] + t, nx);
     };
     auto arm = [&](int g) {  // a pass over group g (6: all rows) begins
-        if (t == 0) vb_arm(bx + 8u * (pass & 1), 4u * (unsigned)A.R.val[g]);
+        if (t == 0 && !dead) vb_arm(bx + 8u * (pass & 1), 4u * (unsigned)A.R.val[g]);
     };
     auto put = [&](unsigned a, float v) {
+        if (dead) return;
         for (int q = 0; q < NC; ++q) vb_send(a, bx + 8u * (pass & 1), R0 + (unsigned)q, v);
     };
     auto send = [&](int row, float v) { put(xb + 4u * (unsigned)row, v); };
@@ -590,7 +619,7 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
         if (cnt == 0 && t == 0) put(smem_u32(&g_word), 0.f);
     };
     auto wait = [&]() {
-        vb_wait(bx + 8u * (pass & 1), (pass >> 1) & 1, A.error, dead);
+        vb_wait(bx + 8u * (pass & 1), (pass >> 1) & 1, A.lim, dead);
         ++pass;
         asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
     };
@@ -609,7 +638,7 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
 #pragma unroll 1
     for (int visit = 0; visit < A.visits; ++visit) {
         if constexpr (ROWS == 0) {
-            if (cg8 && t == 0) vb_arm(bres, 4u * (unsigned)rexp);
+            if (cg8 && t == 0 && !dead) vb_arm(bres, 4u * (unsigned)rexp);
         }
         if (active) {
             fetch(0);
@@ -624,6 +653,7 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
                     vb_row(s, loc + i, w);
                     const float res = __fsub_rn(w.b, __fmaf_rn(x[row0 + i], sdg[loc + i], vb_off(w, x)));
                     const int cd = scd[loc + i];
+                    if (dead) break;
                     if constexpr (ROWS > 0) {
                         vb_send(smem_u32(vsm) + 4u * (unsigned)cd, bres, 0u, res);
                     } else {
@@ -632,11 +662,11 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
                     }
                 }
             }
-            if (t == 0) vb_arm(bxc, 4u * (unsigned)nc);
+            if (t == 0 && !dead) vb_arm(bxc, 4u * (unsigned)nc);
         }
         if constexpr (ROWS == 0) {
             if (cg8) {  // the whole block
-                vb_wait(bres, visit & 1, A.error, dead);
+                vb_wait(bres, visit & 1, A.lim, dead);
                 const int w = t >> 5, l = t & 31;
                 float r[2], cx[2];
 #pragma unroll
@@ -644,16 +674,16 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
                     const float4* c8 = reinterpret_cast<const float4*>(rbuf + 8 * (32 * (w + 8 * q) + l));
                     r[q] = M.row[q] >= 0 ? vb_restrict8(c8[0], c8[1]) : 0.f;
                 }
-                vcg8_solve(A.C, M, cg, (int)rank, R0, r, cx, ph, A.error, dead);
+                vcg8_solve(A.C, M, cg, (int)rank, R0, r, cx, ph, A.lim, dead);
 #pragma unroll
                 for (int q = 0; q < 2; ++q)
-                    if (M.row[q] >= 0)
+                    if (M.row[q] >= 0 && !dead)
                         for (int k = 0; k < NC; ++k)
                             vb_send(smem_u32(xc) + 4u * (unsigned)M.row[q], bxc, (unsigned)k, cx[q]);
             }
         }
         if (!active) continue;
-        vb_wait(bxc, visit & 1, A.error, dead);
+        vb_wait(bxc, visit & 1, A.lim, dead);
         // prolongation: x += x_c of the coarse voxel
         arm(6);
 #pragma unroll 1
@@ -668,8 +698,7 @@ __global__ void __launch_bounds__(VB_THREADS, 1) k_vbottom(VBotArgs A) {
     }
     for (int g = 0; g < 6; ++g)
         for (int i = t; i < g_cnt[g]; i += VB_THREADS) A.lhs[A.R.slot[g_row[g] + i]] = x[g_row[g] + i];
-    __syncthreads();
-    vb_cluster_sync();  // nobody sends into a CTA that has left
+    vb_leave(dead);
 }
 
 }  // namespace uaamg
