@@ -47,3 +47,22 @@ def test_a_wait_that_gives_up_fails_the_solve(gpu, monkeypatch, n, graph):
     for t in (s, s1):
         x = np.zeros_like(rhs)
         assert t.pcg_solve(x, 1e-6, rhs) == st and np.array_equal(x, want)
+
+
+@pytest.mark.parametrize("n", [16, 24])
+def test_calls_outside_a_solve_report_it(gpu, monkeypatch, n):
+    from uaamg_b200._lib import UaamgError
+    lv, s, rhs = make(n)
+    r = np.ones_like(rhs)
+    z, b = s.precondition(r), np.ones((3, lv.leaf_count(lv.num_levels() - 1), 512), np.float32)
+    x = lv.solve_exact(b)
+    monkeypatch.setenv("UAAMG_VISC_WAIT_US", "0")
+    lv0, s0, _ = make(n)
+    with pytest.raises(UaamgError, match="waited too long"):
+        s0.precondition(r)
+    if n == 24:
+        with pytest.raises(UaamgError, match="waited too long"):
+            lv0.solve_exact(b)
+    else:  # one CTA: nothing to wait for, and the error of the call before is not this one's
+        assert np.array_equal(lv0.solve_exact(b), x)
+    assert np.array_equal(s.precondition(r), z) and np.array_equal(lv.solve_exact(b), x)

@@ -1062,6 +1062,22 @@ static void vinit_state(uaamg_viscosity* h) {
     CK(cudaMemcpyAsync(h->st, h->st_host, sizeof(PcgState), cudaMemcpyHostToDevice, h->stream));
 }
 
+// the error word of the state copied back: a bottom cycle or coarsest solve that gave up
+static void vcheck_waits(const uaamg_viscosity* h) {
+    if (!h->st_host->error) return;
+    set_error("the CTAs of a bottom cycle or coarsest solve waited too long for one another");
+    throw UaamgError{UAAMG_ERR_CUDA};
+}
+// Around such launches outside a solve: the word cleared before, read back after them.
+static void vclear_waits(uaamg_viscosity* h) {
+    CK(cudaMemsetAsync(&h->st->error, 0, sizeof(int), h->stream));
+}
+static void vread_waits(uaamg_viscosity* h) {
+    CK(cudaMemcpyAsync(&h->st_host->error, &h->st->error, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    vcheck_waits(h);
+}
+
 // x, b (h->x, h->b) on the device; returns UAAMG_SUCCESS when the stopping
 // test held, UAAMG_FAILED when the loop returned at max_iter - 1
 static int vrun_pcg(uaamg_viscosity* h, std::vector<ProfRec>* prof = nullptr) {
@@ -1120,10 +1136,7 @@ static int vrun_pcg(uaamg_viscosity* h, std::vector<ProfRec>* prof = nullptr) {
     h->last_launches = launches;
     h->launches += launches;
     const PcgState& s = *h->st_host;
-    if (s.error) {
-        set_error("the CTAs of a bottom cycle or coarsest solve waited too long for one another");
-        throw UaamgError{UAAMG_ERR_CUDA};
-    }
+    vcheck_waits(h);
     h->iterations = s.iterations_taken;
     h->final_residual = s.nu;
     h->status = (s.status == PCG_SUCCESS) ? UAAMG_SUCCESS : UAAMG_FAILED;
@@ -1569,10 +1582,11 @@ int uaamg_viscosity_coarsest_solve(uaamg_viscosity* h, const float* rhs, float* 
     float* x = sc.get(vb);
     CK(cudaMemcpyAsync(b, rhs, vb, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemsetAsync(x, 0, vb, h->stream));
+    vclear_waits(h);
     VEnq E{h, h->stream};
     E.coarsest(b, x);
     CK(cudaMemcpyAsync(out, x, vb, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    vread_waits(h);
     return UAAMG_SUCCESS;
     ABI_END
 }
@@ -1586,10 +1600,11 @@ int uaamg_viscosity_precondition(uaamg_viscosity* h, const float* r, float* z) {
     CK(cudaMemcpyAsync(rr, r, vb, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemsetAsync(zz, 0, vb, h->stream));  // a bottom cycle or coarsest solve on level 0 writes the DOF only
     launch2(k_vmask, dim3((unsigned)h->lv[0].L.nl, 3), 128, h->stream, h->lv[0].L, rr);
+    vclear_waits(h);
     VEnq E{h, h->stream};
     enqueue_mucycle(E, 0, zz, rr, true);
     CK(cudaMemcpyAsync(z, zz, vb, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    vread_waits(h);
     return UAAMG_SUCCESS;
     ABI_END
 }
