@@ -1363,6 +1363,7 @@ static bool g_use_bottom = true;
 static bool use_bottom(uaamg_poisson* h) {
     if (h->smoother != UAAMG_SMOOTHER_SCHEDULED_RELAXED_JACOBI && h->smoother != UAAMG_SMOOTHER_WEIGHTED_JACOBI)
         return false;
+    if (!g_tune.bottom_cycle) return false;  // as it is at each solve (g_tune_gen: the graphs follow)
     if (h->bot_state >= 0) return h->bot_state == 1;
     h->bot_state = 0;
     if (h->nlev < 3) return false;
@@ -2046,7 +2047,7 @@ static int create_impl(const uaamg_leaf_grid* liquid_phi, const uaamg_leaf_grid*
         h->st_host = reinterpret_cast<PcgState*>(h->pin_state);
         h->scalar_host = reinterpret_cast<float*>((char*)h->pin_state + ((sizeof(PcgState) + 63) & ~size_t(63)));
         noalloc_resolve(h);
-        h->bot_state = (g_use_bottom && g_tune.bottom_cycle) ? -1 : 0;
+        h->bot_state = g_use_bottom ? -1 : 0;
         h->use_sweep2 = g_use_sweep2;
         {
             int sms = 0;
