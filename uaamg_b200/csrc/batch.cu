@@ -520,6 +520,7 @@ static void bbuild_graph(uaamg_batch* b) {
     cudaGraphConditionalHandle cond;
     CK(cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
     BEnq E{b, b->stream};
+    const CaptureMark mark(b->ctx, b->stream), body_mark(b->ctx, b->body_stream);
     CK(cudaStreamBeginCaptureToGraph(b->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
         benqueue_setup(E, cond, 1);

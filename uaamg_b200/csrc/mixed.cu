@@ -361,6 +361,7 @@ static void mixed_build_graph(uaamg_poisson* h) {
     cudaGraphConditionalHandle cond;
     CK(cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
     Enq S{h, h->stream};
+    const CaptureMark mark(h->ctx, h->stream), body_mark(h->ctx, h->body_stream);
     CK(cudaStreamBeginCaptureToGraph(h->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
         enqueue_setup(S, cond, 1);

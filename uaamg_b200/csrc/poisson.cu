@@ -1788,6 +1788,7 @@ static void build_graph(uaamg_poisson* h) {
     cudaGraphConditionalHandle cond;
     CK(cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
     Enq E{h, h->stream};
+    const CaptureMark mark(h->ctx, h->stream), body_mark(h->ctx, h->body_stream);
     CK(cudaStreamBeginCaptureToGraph(h->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
         enqueue_setup(E, cond, 1);

@@ -15,6 +15,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <unordered_map>
@@ -43,6 +44,8 @@ struct DeviceCtx {
     std::vector<cudaStream_t> streams;
     std::unordered_set<cudaStream_t> own_streams;  // every stream made here; they are never destroyed
     std::vector<std::pair<size_t, void*>> pinned;  // free pinned blocks (capacity, pointer)
+    std::vector<cudaStream_t> capturing;           // streams being captured into the library's own graphs (CaptureMark)
+    cudaStream_t free_stream = nullptr;            // idle blocks go back to the pool on it; nothing else runs there
     std::unordered_map<void*, size_t> live;        // capacity of the blocks in use that may go to `blocks`
     std::vector<FreeBlock> blocks;                 // freed blocks, oldest first
     size_t blocks_bytes = 0;
@@ -74,6 +77,8 @@ inline DeviceCtx* device_ctx(cudaError_t* err) {
         *err = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &thr);
         if (*err != cudaSuccess) { delete c; return nullptr; }
         *err = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
+        if (*err != cudaSuccess) { delete c; return nullptr; }
+        *err = cudaStreamCreateWithFlags(&c->free_stream, cudaStreamNonBlocking);
         if (*err != cudaSuccess) { delete c; return nullptr; }
         ctxs[dev] = c;
     }
@@ -133,7 +138,10 @@ inline void ctx_pinned_release(DeviceCtx* c, void* p, size_t cap) {
 // whose order its reuse is; a block freed as idle for any stream.  Other
 // streams are a caller's, who may destroy them: their frees, and all of a
 // capturing stream's, go to the pool.  At most FREE_BLOCKS_BYTES are kept
-// (the oldest go back to the pool), none when an allocation fails.
+// (the oldest go back to the pool), none when an allocation fails.  A kept
+// block goes back on its own stream, or on free_stream when idle, and stays
+// while that stream is being captured: another thread's graph would take the
+// free in, fail or repeat it.
 inline size_t dev_block_size(size_t bytes) {  // classes 1/8 of a power of two apart, so that similar sizes share blocks
     if (bytes < 1024) return 1024;
     if (bytes > (size_t(64) << 20)) return (bytes + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
@@ -149,15 +157,42 @@ inline bool ctx_capturing(cudaStream_t s) {
     }
     return st != cudaStreamCaptureStatusNone;
 }
-// gives every kept block back to the pool
-inline void ctx_dev_trim(DeviceCtx* c) {
-    std::vector<FreeBlock> out;
-    {
+// A stream that is about to be captured into a graph of the library, until the capture has ended.
+struct CaptureMark {
+    DeviceCtx* c;
+    cudaStream_t s;
+    CaptureMark(DeviceCtx* ctx, cudaStream_t st) : c(ctx), s(st) {
         std::lock_guard<std::mutex> lk(c->mu);
-        out.swap(c->blocks);
-        c->blocks_bytes = 0;
+        c->capturing.push_back(s);
     }
-    for (const FreeBlock& b : out) cudaFreeAsync(b.p, b.s);
+    CaptureMark(const CaptureMark&) = delete;
+    CaptureMark& operator=(const CaptureMark&) = delete;
+    ~CaptureMark() {
+        std::lock_guard<std::mutex> lk(c->mu);
+        c->capturing.erase(std::find(c->capturing.begin(), c->capturing.end(), s));
+    }
+};
+// Gives the oldest kept blocks back to the pool until at most `bytes` in `count` blocks are left; c->mu is held (so that
+// no capture starts meanwhile).  used: receives the streams they were freed on.
+inline cudaError_t ctx_dev_give_back(DeviceCtx* c, size_t bytes, size_t count, std::vector<cudaStream_t>* used = nullptr) {
+    if (c->blocks_bytes <= bytes && c->blocks.size() <= count) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    size_t left = c->blocks.size(), w = 0;
+    for (size_t i = 0; i < c->blocks.size(); ++i) {
+        const FreeBlock b = c->blocks[i];
+        const bool busy = std::find(c->capturing.begin(), c->capturing.end(), b.s) != c->capturing.end();
+        if ((c->blocks_bytes <= bytes && left <= count) || busy || ctx_capturing(b.s)) {
+            c->blocks[w++] = b;
+            continue;
+        }
+        const cudaError_t q = cudaFreeAsync(b.p, b.s);
+        if (q != cudaSuccess) e = q;
+        c->blocks_bytes -= b.cap;
+        --left;
+        if (used && std::find(used->begin(), used->end(), b.s) == used->end()) used->push_back(b.s);
+    }
+    c->blocks.resize(w);
+    return e;
 }
 inline cudaError_t ctx_dev_alloc(DeviceCtx* c, void** p, size_t bytes, cudaStream_t s) {
     const size_t cap = dev_block_size(bytes);
@@ -181,8 +216,12 @@ inline cudaError_t ctx_dev_alloc(DeviceCtx* c, void** p, size_t bytes, cudaStrea
     cudaError_t e = cudaMallocFromPoolAsync(p, cap, c->pool, s);
     if (e == cudaErrorMemoryAllocation && !plain) {
         cudaGetLastError();
-        ctx_dev_trim(c);
-        cudaDeviceSynchronize();
+        {
+            std::lock_guard<std::mutex> lk(c->mu);
+            std::vector<cudaStream_t> used;
+            ctx_dev_give_back(c, 0, 0, &used);
+            for (cudaStream_t u : used) cudaStreamSynchronize(u);
+        }
         e = cudaMallocFromPoolAsync(p, cap, c->pool, s);
     }
     if (e == cudaSuccess && !plain) {
@@ -201,32 +240,19 @@ inline bool ctx_stream_idle(cudaStream_t s) {
 inline cudaError_t ctx_dev_free(DeviceCtx* c, void* p, cudaStream_t s, bool idle = false) {
     if (!p) return cudaSuccess;
     const bool capturing = ctx_capturing(s);
-    std::vector<FreeBlock> out;
     {
         std::lock_guard<std::mutex> lk(c->mu);
         const auto it = c->live.find(p);
         const size_t cap = it == c->live.end() ? 0 : it->second;
         if (cap) c->live.erase(it);
         const bool own = s == nullptr || c->own_streams.count(s) != 0;
-        if (!cap || cap > FREE_BLOCKS_BYTES / 4 || capturing || !(own || (idle && !c->own_streams.empty()))) {
-            out.push_back({p, cap, s, false});
-        } else {
-            c->blocks.push_back({p, cap, own ? s : *c->own_streams.begin(), idle});
+        if (cap && cap <= FREE_BLOCKS_BYTES / 4 && !capturing && (own || idle)) {
+            c->blocks.push_back({p, cap, idle ? c->free_stream : s, idle});
             c->blocks_bytes += cap;
-            size_t n = 0;
-            while (c->blocks_bytes > FREE_BLOCKS_BYTES || c->blocks.size() - n > FREE_BLOCKS_MAX) {
-                out.push_back(c->blocks[n]);
-                c->blocks_bytes -= c->blocks[n++].cap;
-            }
-            c->blocks.erase(c->blocks.begin(), c->blocks.begin() + (ptrdiff_t)n);
+            return ctx_dev_give_back(c, FREE_BLOCKS_BYTES, FREE_BLOCKS_MAX);
         }
     }
-    cudaError_t e = cudaSuccess;
-    for (const FreeBlock& b : out) {
-        const cudaError_t q = cudaFreeAsync(b.p, b.s);
-        if (q != cudaSuccess) e = q;
-    }
-    return e;
+    return cudaFreeAsync(p, s);
 }
 
 }  // namespace uaamg

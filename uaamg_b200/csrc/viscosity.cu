@@ -1013,6 +1013,7 @@ static void vbuild_graph(uaamg_viscosity* h) {
     cudaGraphConditionalHandle cond;
     CK(cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
     VEnq E{h, h->stream};
+    const CaptureMark mark(h->ctx, h->stream), body_mark(h->ctx, h->body_stream);
     CK(cudaStreamBeginCaptureToGraph(h->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
         venqueue_setup(E, cond, 1);
