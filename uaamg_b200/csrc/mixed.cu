@@ -251,7 +251,8 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     const bool staged = g_use_staged && L.nl >= STAGED_MIN_LEAVES;
     const bool split = g_use_staged && L.nl >= SPLIT_MIN_LEAVES;
     int* err = &h->st->error;
-    const bool march = staged && L.nl >= MARCH_MIN_LEAVES_16, march_dot = staged && L.nl >= PIPE_DOT_MIN_LEAVES;
+    const bool march = staged && L.nl >= MARCH_MIN_LEAVES_16;
+    const bool march_dot = g_use_staged && L.nl >= PIPE_DOT_MIN_LEAVES;  // whatever the tuning is
     const int NP = march_planes(L.nl);
     auto sweep = [&](const T* x, T* out, float w) {  // plain source
         if (march)

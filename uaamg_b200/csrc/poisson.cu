@@ -1248,7 +1248,8 @@ struct Enq {
         LevelDev& D = h->lv[l];
         float ws = D.w_sor;
         if constexpr (std::is_same<Src, SrcPlain>::value) {
-            if (g_use_staged && D.L.nl >= STAGED_MIN_LEAVES && !(MODE == M_SPAI0 && mark_spai0)) {
+            const bool large_dot = dot.r && D.L.nl >= PIPE_DOT_MIN_LEAVES;  // marches whatever the tuning is
+            if (g_use_staged && (D.L.nl >= STAGED_MIN_LEAVES || large_dot) && !(MODE == M_SPAI0 && mark_spai0)) {
                 if (prof) pb("L" + std::to_string(l) + " " + mode_name(MODE) + " staged" + (dot.r ? "+dot" : ""));
                 if (D.L.nl >= (dot.r ? DOT_MARCH_MIN_LEAVES : PIPE_MIN_LEAVES)) {
                     auto go = [&](auto kern, int NP) {
@@ -1256,7 +1257,7 @@ struct Enq {
                                      (const float*)nullptr, 0.f);
                     };
                     const int NP = march_planes(D.L.nl, !dot.r);
-                    if (dot.r && D.L.nl < PIPE_DOT_MIN_LEAVES) go(k_march<MODE, DLevel, float, false, 1>, 1);
+                    if (dot.r && !large_dot) go(k_march<MODE, DLevel, float, false, 1>, 1);
                     else if (NP == 8) go(k_march<MODE, DLevel, float, false, 8>, 8);
                     else go(k_march<MODE, DLevel, float, false, 2>, 2);
                 } else
