@@ -17,6 +17,7 @@
 #include "viscosity_bottom.cuh"
 #include "viscosity_build.cuh"
 #include "viscosity_march.cuh"
+#include "viscosity_plain.h"
 
 namespace {
 
@@ -273,7 +274,8 @@ struct VLevelDev {
     float* alt = nullptr;  // second buffer of the fused red-black steps (zero at non-DOF voxel groups), when used
     int* dof_base = nullptr;
     int* org = nullptr;
-    VPlain P{};  // the leaf lists, where the passes take plain leaves apart
+    VPlain P{};  // the leaf lists, where passes take plain leaves apart
+    bool plain_gs[3] = {true, true, true}, plain_restrict = true;  // whether the colours of a channel and the restriction do
 };
 
 }  // namespace
@@ -300,6 +302,7 @@ struct uaamg_viscosity {
     // levels of at least this many leaves take plain leaves apart in every pass (240^3, 2,491 leaves of level 1: 15.3
     // to 13.0 us a colour; a 560-leaf level has 20 plain leaves and gains nothing)
     int plain_min_leaves = 1024;
+    bool plain_always = false;  // UAAMG_VISC_PLAIN_LEAVES is set: every pass of such levels takes them apart
     std::vector<void*> allocs;
     // level-0 construction products kept for the right-hand side
     VolFields V{};
@@ -431,6 +434,10 @@ static void upload_parents(uaamg_viscosity* h, const VHostLevel& H, VLevelDev& D
     D.L.octant = vupload(h, H.octant.data(), H.octant.size());
 }
 
+// The counts of up to PLAIN_HOST_LEVELS levels, in the handle's pinned block behind the PCG state and its scalars (a
+// level has about a fifth of the leaves of the one above).
+constexpr size_t PLAIN_HOST_AT = ((sizeof(PcgState) + 63) & ~size_t(63)) + 192;
+constexpr int PLAIN_HOST_LEVELS = 8;
 // The leaf lists of a level whose passes take plain leaves apart (viscosity_march.cuh).
 static void build_plain(uaamg_viscosity* h, VLevelDev& D) {
     const int nl = D.L.nl;
@@ -449,6 +456,25 @@ static void build_plain(uaamg_viscosity* h, VLevelDev& D) {
     launch2(k_vclass, dim3((unsigned)((nl + 3) / 4)), 128, s, D.L, (const uint32_t*)carr, (const int*)cand, cls, K);
     launch2(k_vlist, dim3(4), 1024, s, nl, (const unsigned char*)cls, list, cnt);
     D.P = VPlain{list, cnt, K};
+}
+// Which passes of the levels with lists use them (viscosity_plain.h): the counts come back with the create's last
+// synchronisation.
+static int* plain_host(uaamg_viscosity* h, int i) { return (int*)((char*)h->pin_state + PLAIN_HOST_AT) + 16 * i; }
+static void plain_counts(uaamg_viscosity* h) {  // before it
+    int i = 0;
+    for (const VLevelDev& D : h->lv)
+        if (D.P.list && i < PLAIN_HOST_LEVELS)
+            CK(cudaMemcpyAsync(plain_host(h, i++), D.P.cnt, 64, cudaMemcpyDeviceToHost, h->stream));
+}
+static void plain_passes(uaamg_viscosity* h) {  // after it
+    if (h->plain_always) return;
+    int i = 0;
+    for (VLevelDev& D : h->lv) {
+        if (!D.P.list || i >= PLAIN_HOST_LEVELS) continue;
+        const int* cnt = plain_host(h, i++);
+        for (int c = 0; c < 3; ++c) D.plain_gs[c] = vplain_colour(D.L.nl, cnt[4 * c + VP_PLAIN], VAPPLY_MINB * g_sms);
+        D.plain_restrict = vplain_restrict(D.L.nl, cnt[12 + VP_PLAIN]);
+    }
 }
 
 // k_vbottom's CG form by the coarsest system's size (rows per thread of a CTA of its own, 0: over eight CTAs)
@@ -716,7 +742,9 @@ static void build_viscosity(uaamg_viscosity* h, const uaamg_leaf_grid* mu_g, con
         CK(cudaMemsetAsync(h->st, 0, sizeof(PcgState), s));
         h->scalar_dev = (float*)((char*)h->st + ((sizeof(PcgState) + 15) & ~size_t(15)));
     }
+    plain_counts(h);
     CK(cudaStreamSynchronize(s));
+    plain_passes(h);
     TRACE("visc trim + coarsest + vectors");
 }
 
@@ -746,7 +774,7 @@ struct VEnq {
         static const char* names[] = {"normal", "residual", "jacobi", "red_gs", "black_gs"};
         if (prof) pb("L" + std::to_string(l) + " " + names[MODE] + (gs ? " c" + std::to_string(c) : std::string()));
         if constexpr (MODE == VM_RED || MODE == VM_BLACK) {
-            if (D.P.list) {
+            if (D.P.list && D.plain_gs[c]) {
                 const dim3 g((unsigned)(VMARCH_MINB * g_sms));
                 if (c == 0) launch2(k_vmarch<MODE, 0>, g, VMARCH_THREADS, s, D.L, D.P, out, b, 1.0f);
                 else if (c == 1) launch2(k_vmarch<MODE, 1>, g, VMARCH_THREADS, s, D.L, D.P, out, b, 1.0f);
@@ -835,7 +863,7 @@ struct VEnq {
     // residual of level l restricted into the rhs of level l + 1 (fused); coarse_lhs (optional) is zeroed
     void residual_restrict(int l, const float* x, const float* b, float* coarse, float* coarse_lhs) {
         if (prof) pb("L" + std::to_string(l) + " residual+restrict");
-        if (h->lv[l].P.list)
+        if (h->lv[l].P.list && h->lv[l].plain_restrict)
             march3<VM_RESTRICT>(l, x, b, VMarchOut{coarse, coarse_lhs, nullptr, nullptr, 0, 0, 0});
         else
             launch2(k_vresrestrict, dim3((unsigned)h->lv[l].L.nl, 3), 128, s, h->lv[l].L, h->lv[l + 1].L, x, b, coarse,
@@ -1252,7 +1280,7 @@ int uaamg_viscosity_create_on_stream(const uaamg_leaf_grid* viscosity, const uaa
         CK(ctx_stream_acquire(h->ctx, &h->own_stream));
         CK(ctx_stream_acquire(h->ctx, &h->body_stream));
         h->stream = stream ? (cudaStream_t)stream : h->own_stream;
-        CK(ctx_pinned_acquire(h->ctx, sizeof(PcgState) + 256, &h->pin_state, &h->pin_state_cap));
+        CK(ctx_pinned_acquire(h->ctx, PLAIN_HOST_AT + 64 * PLAIN_HOST_LEVELS, &h->pin_state, &h->pin_state_cap));
         h->st_host = reinterpret_cast<PcgState*>(h->pin_state);
         h->scalar_host = reinterpret_cast<float*>((char*)h->pin_state + ((sizeof(PcgState) + 63) & ~size_t(63)));
         {
@@ -1265,7 +1293,10 @@ int uaamg_viscosity_create_on_stream(const uaamg_leaf_grid* viscosity, const uaa
         if (const char* e = getenv("UAAMG_VISC_FUSED_RB_LEAVES")) h->rb_fused_max_leaves = atoi(e);
         if (const char* e = getenv("UAAMG_VISC_SEQ_LEAVES")) h->seq_min_leaves = atoi(e);
         if (const char* e = getenv("UAAMG_VISC_WAIT_US")) h->wait_ns = 1000ull * std::min(std::max(atol(e), 0L), 10000000L);
-        if (const char* e = getenv("UAAMG_VISC_PLAIN_LEAVES")) h->plain_min_leaves = atoi(e);
+        if (const char* e = getenv("UAAMG_VISC_PLAIN_LEAVES")) {
+            h->plain_min_leaves = atoi(e);
+            h->plain_always = true;
+        }
         build_viscosity(h, viscosity, liquid_sdf, solid_sdf, dt, rho, dx);
     } catch (const UaamgError& e) {
         uaamg_viscosity_destroy(h);
