@@ -8,7 +8,6 @@ import subprocess
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-WAVE = 7 * 148
 
 
 @pytest.fixture(scope="module")
@@ -17,7 +16,7 @@ def rule(tmp_path_factory):
     src, lib = d / "shim.cpp", d / "shim.so"
     src.write_text('#include "viscosity_plain.h"\nextern "C" {\n'
                    "int restrict_(int nl, int plain) { return uaamg::vplain_restrict(nl, plain); }\n"
-                   "int colour(int nl, int plain, int wave) { return uaamg::vplain_colour(nl, plain, wave); }\n}\n")
+                   "int colour(int nl, int plain) { return uaamg::vplain_colour(nl, plain); }\n}\n")
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "uaamg_b200", "csrc"), "-o", str(lib),
                     str(src)], check=True)
     return C.CDLL(str(lib))
@@ -43,7 +42,7 @@ def test_restriction(rule, nl, plain, lists, general):
 
 @pytest.mark.parametrize("nl,plain,lists,general", COLOUR)
 def test_colour(rule, nl, plain, lists, general):
-    took, other = (lists, general) if rule.colour(nl, plain, WAVE) else (general, lists)
+    took, other = (lists, general) if rule.colour(nl, plain) else (general, lists)
     assert took <= 1.01 * other
 
 
@@ -51,5 +50,5 @@ def test_no_plain_leaves(rule):
     """What the lists cost where nothing is plain is not paid."""
     for nl in range(1024, 40000, 7):
         assert not rule.restrict_(nl, 0)
-        assert nl >= 4096 or not rule.colour(nl, 0, WAVE)
-        assert rule.restrict_(nl, nl) and rule.colour(nl, nl, WAVE)
+        assert nl >= 4096 or not rule.colour(nl, 0)
+        assert rule.restrict_(nl, nl) and rule.colour(nl, nl)

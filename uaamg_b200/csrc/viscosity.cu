@@ -472,7 +472,7 @@ static void plain_passes(uaamg_viscosity* h) {  // after it
     for (VLevelDev& D : h->lv) {
         if (!D.P.list || i >= PLAIN_HOST_LEVELS) continue;
         const int* cnt = plain_host(h, i++);
-        for (int c = 0; c < 3; ++c) D.plain_gs[c] = vplain_colour(D.L.nl, cnt[4 * c + VP_PLAIN], VAPPLY_MINB * g_sms);
+        for (int c = 0; c < 3; ++c) D.plain_gs[c] = vplain_colour(D.L.nl, cnt[4 * c + VP_PLAIN]);
         D.plain_restrict = vplain_restrict(D.L.nl, cnt[12 + VP_PLAIN]);
     }
 }

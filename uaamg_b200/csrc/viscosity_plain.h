@@ -1,8 +1,9 @@
 // viscosity_plain.h -- which passes of a viscosity level take its plain leaves
 // apart (viscosity_march.cuh), by how many it has.  Host, without CUDA.
 //
-// The passes over both kinds run four CTAs per SM, so a level with few plain
-// leaves gives up warps for nothing: the general kernels hold seven.  q = A x
+// The passes over both kinds have four CTAs per SM and 128 registers a thread;
+// the general kernels, three CTAs with up to 168, hold more of a general leaf's
+// loads in flight, which is what a level with few plain leaves needs.  q = A x
 // and the first residual gain all the same (leaves without DOFs are skipped).
 // Whole solves with viscosity that varies in part of the domain, ms, lists /
 // general kernel, by leaves and plain leaves of the level:
@@ -19,16 +20,17 @@
 namespace uaamg {
 
 constexpr int VPLAIN_LARGE = 4096;  // levels of this many leaves: bytes bound both forms
+constexpr int VPLAIN_SMALL = 1280;  // levels below: a CTA has one or two leaves in all
 constexpr int VPLAIN_RESTRICT = 512;  // plain leaves from which a smaller level's restriction gains
 
 // residual + restriction; plain: leaves plain in every channel
 inline bool vplain_restrict(int nl, int plain) {
     return nl >= VPLAIN_LARGE ? plain >= nl / 32 : plain >= VPLAIN_RESTRICT;
 }
-// a colour of a channel; plain: leaves plain in that channel; wave: leaves the general kernel holds at once
-inline bool vplain_colour(int nl, int plain, int wave) {
+// a colour of a channel; plain: leaves plain in that channel
+inline bool vplain_colour(int nl, int plain) {
     if (nl >= VPLAIN_LARGE) return true;
-    return nl <= wave + wave / 4 ? plain >= nl / 6 : plain >= nl / 32;
+    return plain >= (nl < VPLAIN_SMALL ? nl / 6 : nl / 32);
 }
 
 }  // namespace uaamg
