@@ -358,7 +358,7 @@ class PoissonBytes:
         if l >= len(self.levels):
             return None
         n = float(self.levels[l][0])
-        kind = " ".join(parts[1:]).replace(" staged", "")
+        kind = " ".join(parts[1:]).replace(" staged", "").replace(" march", "")
         dot = 4.0 * n if kind.endswith("+dot") else 0.0
         kind = kind.replace("+dot", "")
         if kind == "jacobi":                     # x, b, out + coefficients and 1/diag
@@ -385,8 +385,9 @@ class PoissonBytes:
     def ncu_tag(label: str, leaves: int) -> str:
         """The kernel name and level size the committed ncu summaries use for
         this class (a kernel's traffic depends on the level it sweeps)."""
-        if "jacobi staged" in label and "+dot" not in label:
-            return f"k_sweep_staged<0> ({leaves} leaves)"
+        for kind, kernel in (("jacobi march", "k_march<0>"), ("jacobi staged", "k_sweep_staged<0>")):
+            if kind in label and "+dot" not in label:
+                return f"{kernel} ({leaves} leaves)"
         return label
 
 
@@ -492,11 +493,11 @@ def run_viscosity(args, dev, stream, timed, max_over_ranks, ws, rank, vsc, vdg, 
            "step": "create viscosity matrix+hierarchy, rhs, warm start, UAAMG-PCG",
            "solves_per_s": round(1e3 / value, 2),
            "roofline": {"bound": "hbm",
-                        "kernel": f"k_vapply_seq<RED_GS> level 0, channel 0 ({n0} leaves over 3 CTAs per SM)",
+                        "kernel": f"k_vmarch<RED_GS> level 0, channel 0 ({n0} leaves, 4 CTAs per SM)",
                         "achieved": round(achieved, 1) if achieved else None, "peak": peak,
                         "peak_kind": peak_kind, "unit": "GB/s",
                         "frac": round(achieved / peak, 4) if achieved else None,
-                        "traffic": _traffic_from_profile("k_vapply_seq<3>"), "algorithmic_bytes_per_launch": dom_bytes,
+                        "traffic": _traffic_from_profile(f"k_vmarch<3> ({n0} leaves)"), "algorithmic_bytes_per_launch": dom_bytes,
                         "avg_launch_us": round(t_ms / cnt * 1e3, 2) if cnt else None,
                         "level0_rbgs_GBps": round(l0_bytes / (l0_ms * 1e-3) / 1e9, 1) if l0_ms else None,
                         "all_levels_rbgs_GBps": round(gs_bytes / (gs_ms * 1e-3) / 1e9, 1) if gs_ms else None,

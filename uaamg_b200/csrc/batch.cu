@@ -20,7 +20,7 @@
 // Every CTA runs the same per-leaf device code as the single-instance
 // kernels, and each reduction keeps the instance's leaf slots and order, so
 // each instance's result, iteration count and status are bit-identical to its
-// standalone solve.  From PIPE_DOT_MIN_LEAVES leaves on a standalone solve adds
+// standalone solve.  From DOT_MARCH_LARGE_LEAVES leaves on a standalone solve adds
 // its dot products in another order (a partial per CTA of k_march, here one per
 // leaf): FP64 sums, equal once rounded to the FP32 scalars of the CG unless a
 // sum lies within some 1e-15 of where that rounding turns.

@@ -212,7 +212,7 @@ struct MEnq {
 // SPLIT_MIN_LEAVES on the first sweep's source and the prolongation-add are
 // stored first (k_mmaterialize) so that every sweep is a staged plain one.
 // 16-bit levels march from this size on (smaller ones: the one-leaf staged
-// kernels, as at PIPE_MIN_LEAVES).
+// kernels, as at MARCH_MIN_LEAVES).
 #define MARCH_MIN_LEAVES_16 1024
 template <typename T>
 static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
@@ -252,11 +252,11 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     const bool split = g_use_staged && L.nl >= SPLIT_MIN_LEAVES;
     int* err = &h->st->error;
     const bool march = staged && L.nl >= MARCH_MIN_LEAVES_16;
-    const bool march_dot = g_use_staged && L.nl >= PIPE_DOT_MIN_LEAVES;  // whatever the tuning is
+    const bool march_dot = g_use_staged && L.nl >= DOT_MARCH_LARGE_LEAVES;  // whatever the tuning is
     const int NP = march_planes(L.nl);
     auto sweep = [&](const T* x, T* out, float w) {  // plain source
         if (march)
-            E.run_march("jacobi staged", l, NP, NP == 8 ? k_march<M_JACOBI, MLevel<T>, T, false, 8>
+            E.run_march("jacobi march", l, NP, NP == 8 ? k_march<M_JACOBI, MLevel<T>, T, false, 8>
                                                         : k_march<M_JACOBI, MLevel<T>, T, false, 2>,
                         L.nl, L, x, (const T*)rhs, out, w, 0.f, 0.f, nodot, ns, 0.f);
         else if (staged)
@@ -283,7 +283,7 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     const float cics = 1.0f / level_scale(h->lv[l + 1].L);
     T* crhs = (T*)M->lv[l + 1].rhs;
     if (march)  // the marching kernel computes in stored units: its scale is cs / cs'
-        E.run_march("restrict staged", l, NP, NP == 8 ? k_march<M_RESIDUAL, MLevel<T>, T, true, 8>
+        E.run_march("restrict march", l, NP, NP == 8 ? k_march<M_RESIDUAL, MLevel<T>, T, true, 8>
                                                       : k_march<M_RESIDUAL, MLevel<T>, T, true, 2>,
                     L.nl, L, (const T*)tmp, (const T*)rhs, crhs, 0.f, 0.f, 0.f, nodot, ns, L.cs * cics);
     else if (staged)
@@ -304,7 +304,7 @@ static void menq_visit(MEnq& E, int l, bool skip_first, DotOut dot, float* z) {
     sweep(lhs, tmp, wpre(1));
     if (l == 0) {
         if (march_dot)
-            E.run_march("jacobi staged to fp32 +dot", l, NP, NP == 8 ? k_march<M_JACOBI, MLevel<T>, float, false, 8>
+            E.run_march("jacobi march to fp32 +dot", l, NP, NP == 8 ? k_march<M_JACOBI, MLevel<T>, float, false, 8>
                                                                      : k_march<M_JACOBI, MLevel<T>, float, false, 2>,
                         L.nl, L, (const T*)tmp, (const T*)rhs, z, wpre(0), 0.f, 0.f, dot, (const float*)M->sigma, 0.f);
         else if (staged)

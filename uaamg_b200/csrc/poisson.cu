@@ -1021,12 +1021,12 @@ static int g_sms = 148;  // SMs of the device (set when a handle is created)
 // stored values are the ones the fused kernel computes, so the results are
 // identical.
 #define SPLIT_MIN_LEAVES (g_tune.split_min_leaves)
-// Sweeps of a stored source march from PIPE_MIN_LEAVES leaves on
+// Sweeps of a stored source march from MARCH_MIN_LEAVES leaves on
 // (poisson_march.cuh); smaller staged levels use the one-leaf staged kernels,
 // whose four times as many warps hide more of a small level's latency.
 // Measured, Jacobi, marching / staged: 1,916 leaves 9.2 / 10.2 us, 284 leaves
 // 7.9 / 7.9 us.  Residual + restriction marches on every staged level.
-#define PIPE_MIN_LEAVES (g_tune.pipe_min_leaves)
+#define MARCH_MIN_LEAVES (g_tune.pipe_min_leaves)
 // Planes a half-warp marches: two (four times the warps, each plane along x
 // read twice) or a whole leaf.  A pass that ends in a reduction or stores an
 // eighth gains from fewer warps first, a 16-bit one as well; an FP32 sweep only
@@ -1036,14 +1036,14 @@ static int g_sms = 148;  // SMs of the device (set when a handle is created)
 // 187 / 177; 16-bit sweep at 30,492: 54 / 49.
 static int march_planes(int nl, bool fp32_sweep = false) { return nl >= (fp32_sweep ? 65536 : 24576) ? 8 : 2; }
 // A pass that carries a level-0 dot product (the last post-smoothing sweep
-// with z.r, A p with p.q) marches two or eight planes from PIPE_DOT_MIN_LEAVES
+// with z.r, A p with p.q) marches two or eight planes from DOT_MARCH_LARGE_LEAVES
 // leaves on: its per-CTA partials set the dot's summation order, which must not
 // depend on the tuning.  Below, from DOT_MARCH_MIN_LEAVES on, a leaf per CTA
 // and a plane per half-warp: a thread then holds the voxels it holds in the
 // one-leaf kernels and the sums are theirs (6,400 leaves, one-leaf / marching:
 // A p 21 / 19 us, sweep 21 / 19; 1,916 leaves: 16.8 / 14.8, 16.8 / 16.8).  The
-// mixed-precision form marches its dot from PIPE_DOT_MIN_LEAVES on.
-#define PIPE_DOT_MIN_LEAVES 8192
+// mixed-precision form marches its dot from DOT_MARCH_LARGE_LEAVES on.
+#define DOT_MARCH_LARGE_LEAVES 8192
 #define DOT_MARCH_MIN_LEAVES 1024
 // Grid of the grid-stride elementwise kernels (k_materialize, the PCG
 // vector updates): 16 CTAs of 128 threads per SM of a 148-SM B200, at most
@@ -1248,10 +1248,12 @@ struct Enq {
         LevelDev& D = h->lv[l];
         float ws = D.w_sor;
         if constexpr (std::is_same<Src, SrcPlain>::value) {
-            const bool large_dot = dot.r && D.L.nl >= PIPE_DOT_MIN_LEAVES;  // marches whatever the tuning is
+            const bool large_dot = dot.r && D.L.nl >= DOT_MARCH_LARGE_LEAVES;  // marches whatever the tuning is
             if (g_use_staged && (D.L.nl >= STAGED_MIN_LEAVES || large_dot) && !(MODE == M_SPAI0 && mark_spai0)) {
-                if (prof) pb("L" + std::to_string(l) + " " + mode_name(MODE) + " staged" + (dot.r ? "+dot" : ""));
-                if (D.L.nl >= (dot.r ? DOT_MARCH_MIN_LEAVES : PIPE_MIN_LEAVES)) {
+                const bool march = D.L.nl >= (dot.r ? DOT_MARCH_MIN_LEAVES : MARCH_MIN_LEAVES);
+                if (prof)
+                    pb("L" + std::to_string(l) + " " + mode_name(MODE) + (march ? " march" : " staged") + (dot.r ? "+dot" : ""));
+                if (march) {
                     auto go = [&](auto kern, int NP) {
                         launch_march(kern, D.L.nl, NP, s, D.L, (const float*)src.x, b, out, w, ws, 1.0f - ws, dot,
                                      (const float*)nullptr, 0.f);
@@ -1307,7 +1309,7 @@ struct Enq {
     void restrict_resid(int l, const float* x, const float* b) {
         LevelDev& D = h->lv[l];
         if (g_use_staged && D.L.nl >= STAGED_MIN_LEAVES) {
-            if (prof) pb("L" + std::to_string(l) + " residual+restrict staged");
+            if (prof) pb("L" + std::to_string(l) + " residual+restrict march");
             auto go = [&](auto kern, int NP) {
                 launch_march(kern, D.L.nl, NP, s, D.L, x, b, h->lv[l + 1].rhs, 0.f, 0.f, 0.f,
                              DotOut{nullptr, nullptr, nullptr}, (const float*)nullptr, 0.f);
@@ -1647,7 +1649,7 @@ static void enqueue_setup(Enq& E, cudaGraphConditionalHandle cond, int use_cond)
 static void enqueue_Ap(Enq& E) {
     uaamg_poisson* h = E.h;
     LevelDev& D0 = h->lv[0];
-    const bool large = D0.L.nl >= PIPE_DOT_MIN_LEAVES;
+    const bool large = D0.L.nl >= DOT_MARCH_LARGE_LEAVES;
     if (g_use_staged && (large || D0.L.nl >= std::max(DOT_MARCH_MIN_LEAVES, (int)STAGED_MIN_LEAVES))) {
         const int NP = large ? march_planes(D0.L.nl) : 1;
         launch_march(NP == 8   ? k_march<M_LAPLACIAN, DLevel, float, false, 8, 1>

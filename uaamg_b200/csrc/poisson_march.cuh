@@ -30,8 +30,8 @@
 namespace uaamg {
 
 // ---- storage element traits
-template <typename E> struct PipeE;
-template <> struct PipeE<float> {
+template <typename E> struct MarchE;
+template <> struct MarchE<float> {
     static __device__ __forceinline__ float4 q(const float* p) { return *reinterpret_cast<const float4*>(p); }
     static __device__ __forceinline__ float v(const float* p) { return *p; }
     static __device__ __forceinline__ void st(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
@@ -47,8 +47,8 @@ template <> struct PipeE<float> {
 // and the product with the stored 1/diag is the true value -- with the defaults
 // of trimmed leaves brought to the same units (def_face / cs, def_diag / cs,
 // def_invdiag * cs).  Each result equals the one computed from rescaled values.
-template <class LV> struct PipeLv;
-template <> struct PipeLv<DLevel> {
+template <class LV> struct MarchLv;
+template <> struct MarchLv<DLevel> {
     using E = float;
     static constexpr bool SCALED = false;
     static __device__ __forceinline__ float def_face(const DLevel& L) { return L.def_face; }
@@ -139,12 +139,12 @@ __host__ __device__ __forceinline__ unsigned march_grid(int nl, int NP) {
 // dot.r, 1 p.q with p the swept vector.
 template <int MODE, class LV, typename TOut, bool RESTRICT, int NP, int DOTK = 0>
 __device__ __forceinline__ double march_leaf(const LV& L, int leaf, int X0, bool on,
-                                             const typename PipeLv<LV>::E* x, const typename PipeLv<LV>::E* b, TOut* out,
+                                             const typename MarchLv<LV>::E* x, const typename MarchLv<LV>::E* b, TOut* out,
                                              float w, float wsor, float one_minus_wsor, const DotOut& dot,
                                              const float* zscale, float coarse_scale, const unsigned* gate = nullptr) {
-    using T = PipeLv<LV>;
+    using T = MarchLv<LV>;
     using E = typename T::E;
-    using P = PipeE<E>;
+    using P = MarchE<E>;
     const int lane = threadIdx.x & 31, q = lane & 15, Y = q >> 1, zh = q & 1;
     const long long l0 = (long long)leaf * UAAMG_LEAF;
     // ---- static data, before the wait for the previous kernel
@@ -217,13 +217,13 @@ __device__ __forceinline__ double march_leaf(const LV& L, int leaf, int X0, bool
                     s[k] = __fmul_rn(a, 0.125f);
                     if (T::SCALED) s[k] = __fmul_rn(s[k], coarse_scale);
                 }
-                if (on && (Y & 1) == 0) PipeE<TOut>::st2(po + 64 * (i >> 1), s[0], s[1]);
+                if (on && (Y & 1) == 0) MarchE<TOut>::st2(po + 64 * (i >> 1), s[0], s[1]);
             }
         } else {
             if constexpr (T::SCALED) {
                 if (zscale) res = f4mul(res, *zscale);
             }
-            if (on) PipeE<TOut>::st(po + 64 * i, res);
+            if (on) MarchE<TOut>::st(po + 64 * i, res);
             if (dot.r) {  // z.r or p.q
                 float4 rr = DOTK == 1 ? xc : bb;
                 if constexpr (T::SCALED && DOTK == 0) rr = ld4(dot.r, leaf, (X0 + i) * 16 + q);
@@ -347,8 +347,8 @@ __device__ __forceinline__ void march_dot(double sum, const DotOut& dot, int slo
 // 13-15, DOTK 0), or sigma and alpha (lines 6-7, DOTK 1); a partial per CTA, in
 // an order that depends on the level only (NP 1: a CTA is a leaf, its threads those of the one-leaf kernels).
 template <int MODE, class LV, typename TOut, bool RESTRICT, int NP, int DOTK = 0>
-__global__ void __launch_bounds__(MARCH_THREADS, PipeLv<LV>::SCALED ? MARCH_MINB16 : MARCH_MINB)
-    k_march(LV L, const typename PipeLv<LV>::E* x, const typename PipeLv<LV>::E* b, TOut* out, float w, float wsor,
+__global__ void __launch_bounds__(MARCH_THREADS, MarchLv<LV>::SCALED ? MARCH_MINB16 : MARCH_MINB)
+    k_march(LV L, const typename MarchLv<LV>::E* x, const typename MarchLv<LV>::E* b, TOut* out, float w, float wsor,
             float one_minus_wsor, DotOut dot, const float* zscale, float coarse_scale) {
     constexpr int SEG = 8 / NP;
     const long long item = (long long)blockIdx.x * (MARCH_THREADS / 16) + (threadIdx.x >> 4);

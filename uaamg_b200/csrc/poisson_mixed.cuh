@@ -114,7 +114,7 @@ __device__ __forceinline__ float4 ldi4(const MLevel<T>& L, long long leaf, int t
 
 // storage and level traits of the marching sweeps (poisson_march.cuh)
 template <typename T>
-struct PipeE16 {
+struct MarchE16 {
     static __device__ __forceinline__ float4 q(const T* p) { return ldh4(p, 0, 0); }
     static __device__ __forceinline__ float v(const T* p) { return H16<T>::to1(*p); }
     static __device__ __forceinline__ void st(T* p, float4 v) { sth4(p, 0, 0, v); }
@@ -122,10 +122,10 @@ struct PipeE16 {
         *reinterpret_cast<unsigned*>(p) = H16<T>::from2(a, b);
     }
 };
-template <> struct PipeE<__half> : PipeE16<__half> {};
-template <> struct PipeE<__nv_bfloat16> : PipeE16<__nv_bfloat16> {};
+template <> struct MarchE<__half> : MarchE16<__half> {};
+template <> struct MarchE<__nv_bfloat16> : MarchE16<__nv_bfloat16> {};
 template <typename T>
-struct PipeLv<MLevel<T>> {  // computes in stored units (poisson_march.cuh)
+struct MarchLv<MLevel<T>> {  // computes in stored units (poisson_march.cuh)
     using E = T;
     static constexpr bool SCALED = true;
     static __device__ __forceinline__ float def_face(const MLevel<T>& L) { return __fmul_rn(L.def_face, L.ics); }
