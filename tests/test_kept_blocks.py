@@ -24,6 +24,7 @@ std::unordered_map<void*, size_t> out;      // blocks the pool has given
 std::set<cudaStream_t> captured;            // as cudaStreamIsCapturing sees it
 size_t used = 0, total = ~size_t(0), next = 4096, streams = 256;
 int bad_frees = 0, device_syncs = 0;
+std::unordered_map<void*, cudaStream_t> freed;  // where each block last went back
 }
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
@@ -51,6 +52,7 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t s) {
     bad_frees += captured.count(s) || !out.count(p);
     used -= out[p];
     out.erase(p);
+    freed[p] = s;
     return cudaSuccess;
 }
 static DeviceCtx* ctx() { cudaError_t e; return device_ctx(&e); }
@@ -66,6 +68,8 @@ void k_total(size_t n) { total = n; }
 size_t k_used() { return used; }
 size_t k_kept() { return ctx()->blocks_bytes; }
 size_t k_blocks() { return ctx()->blocks.size(); }
+long k_freed(long p) { return freed.count((void*)p) ? (long)freed[(void*)p] : -1; }
+long k_free_stream() { return (long)ctx()->free_stream; }
 int k_bad() { return bad_frees; }
 int k_device_syncs() { return device_syncs; }
 }
@@ -81,10 +85,11 @@ def k(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-O1", "-fno-gnu-unique", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", cuda, "-I",
                     os.path.join(ROOT, "uaamg_b200", "csrc"), "-o", str(lib), str(src)], check=True)
     f = C.CDLL(str(lib))
-    for name in ("k_stream", "k_alloc", "k_used", "k_kept", "k_blocks"):
+    for name in ("k_stream", "k_alloc", "k_used", "k_kept", "k_blocks", "k_freed", "k_free_stream"):
         getattr(f, name).restype = C.c_size_t
     f.k_alloc.argtypes = [C.c_size_t, C.c_long]
     f.k_free.argtypes = [C.c_long, C.c_long, C.c_int]
+    f.k_freed.argtypes = [C.c_long]
     f.k_captured.argtypes = [C.c_long, C.c_int]
     f.k_mark.argtypes, f.k_mark.restype, f.k_unmark.argtypes = [C.c_long], C.c_void_p, [C.c_void_p]
     f.k_total.argtypes = [C.c_size_t]
@@ -175,3 +180,25 @@ def test_an_allocation_that_fails_gets_what_is_kept(k):
     k.k_captured(b, 0)
     assert k.k_alloc(420 << 20, a) != 0
     assert k.k_blocks() == 0
+
+
+@pytest.mark.parametrize("idle", [0, 1])
+@pytest.mark.parametrize("captured", [0, 1])
+def test_where_blocks_go_back(k, captured, idle):
+    """On the stream they were freed on, whose later allocations the pool can
+    serve from them at once; an idle block of a captured stream or of a caller's
+    on the stream kept for that."""
+    a, b = k.k_stream(), k.k_stream()
+    p, q = k.k_alloc(300 << 20, a), k.k_alloc(301 << 20, CALLER)
+    k.k_free(p, a, idle)
+    k.k_free(q, CALLER, 1)
+    k.k_captured(a, captured)
+    for r in [k.k_alloc((400 + i) << 20, b) for i in range(6)]:
+        k.k_free(r, b, 0)
+    assert k.k_freed(q) == k.k_free_stream()
+    if not captured:
+        assert k.k_freed(p) == a
+    elif idle:
+        assert k.k_freed(p) == k.k_free_stream()
+    else:
+        assert k.k_freed(p) == C.c_size_t(-1).value  # kept

@@ -45,7 +45,7 @@ struct DeviceCtx {
     std::unordered_set<cudaStream_t> own_streams;  // every stream made here; they are never destroyed
     std::vector<std::pair<size_t, void*>> pinned;  // free pinned blocks (capacity, pointer)
     std::vector<cudaStream_t> capturing;           // streams being captured into the library's own graphs (CaptureMark)
-    cudaStream_t free_stream = nullptr;            // idle blocks go back to the pool on it; nothing else runs there
+    cudaStream_t free_stream = nullptr;            // where idle blocks of no usable stream go back; nothing else runs there
     std::unordered_map<void*, size_t> live;        // capacity of the blocks in use that may go to `blocks`
     std::vector<FreeBlock> blocks;                 // freed blocks, oldest first
     size_t blocks_bytes = 0;
@@ -139,9 +139,10 @@ inline void ctx_pinned_release(DeviceCtx* c, void* p, size_t cap) {
 // streams are a caller's, who may destroy them: their frees, and all of a
 // capturing stream's, go to the pool.  At most FREE_BLOCKS_BYTES are kept
 // (the oldest go back to the pool), none when an allocation fails.  A kept
-// block goes back on its own stream, or on free_stream when idle, and stays
-// while that stream is being captured: another thread's graph would take the
-// free in, fail or repeat it.
+// block goes back on the stream it was freed on, where the pool can reuse it at
+// once.  While that stream is being captured it must not (another thread's
+// graph would take the free in, fail or repeat it): an idle block then goes
+// back on free_stream, any other stays.
 inline size_t dev_block_size(size_t bytes) {  // classes 1/8 of a power of two apart, so that similar sizes share blocks
     if (bytes < 1024) return 1024;
     if (bytes > (size_t(64) << 20)) return (bytes + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
@@ -179,9 +180,13 @@ inline cudaError_t ctx_dev_give_back(DeviceCtx* c, size_t bytes, size_t count, s
     cudaError_t e = cudaSuccess;
     size_t left = c->blocks.size(), w = 0;
     for (size_t i = 0; i < c->blocks.size(); ++i) {
-        const FreeBlock b = c->blocks[i];
-        const bool busy = std::find(c->capturing.begin(), c->capturing.end(), b.s) != c->capturing.end();
-        if ((c->blocks_bytes <= bytes && left <= count) || busy || ctx_capturing(b.s)) {
+        FreeBlock b = c->blocks[i];
+        bool keep = c->blocks_bytes <= bytes && left <= count;
+        if (!keep && (std::find(c->capturing.begin(), c->capturing.end(), b.s) != c->capturing.end() || ctx_capturing(b.s))) {
+            if (b.idle) b.s = c->free_stream;
+            else keep = true;
+        }
+        if (keep) {
             c->blocks[w++] = b;
             continue;
         }
@@ -247,7 +252,7 @@ inline cudaError_t ctx_dev_free(DeviceCtx* c, void* p, cudaStream_t s, bool idle
         if (cap) c->live.erase(it);
         const bool own = s == nullptr || c->own_streams.count(s) != 0;
         if (cap && cap <= FREE_BLOCKS_BYTES / 4 && !capturing && (own || idle)) {
-            c->blocks.push_back({p, cap, idle ? c->free_stream : s, idle});
+            c->blocks.push_back({p, cap, own ? s : c->free_stream, idle});
             c->blocks_bytes += cap;
             return ctx_dev_give_back(c, FREE_BLOCKS_BYTES, FREE_BLOCKS_MAX);
         }
